@@ -254,24 +254,31 @@ struct BtStep5 {
     }
 };
 
+// Tile of the FP64 product steps: 16 x 16 outputs, one per thread.  The operands have 48-204 rows and
+// 24-51 columns, of which a 64 x 64 tile pads up to half with FP64 instructions, and a few instances
+// do not fill the SMs with larger tiles.  8 / 64 acenes, 4 LE + 1 CT roots, wall time per call:
+// 64 x 64 19.5 / 103.8 ms, 32 x 32 13.5 / 83.2, 16 x 16 11.6 / 71.4, 8 x 16 11.1 / 72.0 (its tile
+// tables are twice as long on the host).
+using BtTile = F64T16;
+
 template <bool TA, bool TB, class Step>
-__global__ void __launch_bounds__(GB_T) bt_gemm_kernel(const int4 *__restrict__ tiles, Step step) {
-    __shared__ double As[GB_K][GB_M + 1];
-    __shared__ double Bs[GB_K][GB_N + 1];
+__global__ void __launch_bounds__(BtTile::T) bt_gemm_kernel(const int4 *__restrict__ tiles, Step step) {
+    __shared__ double As[BtTile::KS][BtTile::M + 1];
+    __shared__ double Bs[BtTile::KS][BtTile::N + 1];
     const int4 t = tiles[blockIdx.x];
     BtOp op;
     if (!step.setup(t.x, t.y, op)) return;   // uniform over the CTA
-    const int m0 = t.z * GB_M, n0 = t.w * GB_N;
-    double acc[4][4];
-    gemm_f64_tile<TA, TB>(op.M, op.N, 0, op.K, op.A, op.lda, op.B, op.ldb, m0, n0, As, Bs, acc);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int m0 = t.z * BtTile::M, n0 = t.w * BtTile::N;
+    double acc[BtTile::O][BtTile::O];
+    f64_tile<BtTile, TA, TB>(op.M, op.N, 0, op.K, op.A, op.lda, op.B, op.ldb, m0, n0, As, Bs, acc);
+    const int tx = threadIdx.x % BtTile::X, ty = threadIdx.x / BtTile::X;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty + 16 * i;
+    for (int i = 0; i < BtTile::O; ++i) {
+        const int m = m0 + ty + BtTile::Y * i;
         if (m >= op.M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 16 * j;
+        for (int j = 0; j < BtTile::O; ++j) {
+            const int n = n0 + tx + BtTile::X * j;
             if (n < op.N) step.epi(op, m, n, acc[i][j]);
         }
     }
@@ -1412,7 +1419,7 @@ static void bt_launch(Ctx &c, cudaStream_t st, const DevBuf<int4> &tiles, size_t
                       double flops) {
     if (n_tiles == 0) return;
     int slot = c.prof_begin(family);
-    bt_gemm_kernel<TA, TB, Step><<<(unsigned)n_tiles, GB_T, 0, st>>>(tiles.p, step);
+    bt_gemm_kernel<TA, TB, Step><<<(unsigned)n_tiles, BtTile::T, 0, st>>>(tiles.p, step);
     count_launch(st, "bt_gemm");
     check_launch("bt_gemm");
     c.prof_end(slot, flops, 0.0);
@@ -1827,27 +1834,28 @@ int Ctx::solve_batch(int n_inst, const tincr_tda_instance *hin, int max_iter, do
     for (int I = 0; I < n_inst; ++I) {
         const BtInst &b = w.h[I];
         const int n2 = 2 * b.n, g = I < g_lo[1] ? 0 : 1;
-        for (int tm = 0; tm < ceil_div(b.n, GB_M); ++tm)
-            for (int tn = 0; tn < ceil_div(b.o + b.v, GB_N); ++tn) tsc.push_back(make_int4(I, 0, tm, tn));
+        const int sc_m = fp64_products ? BtTile::M : GB_M, sc_n = fp64_products ? BtTile::N : GB_N;   // bt_sc32: 64 x 64
+        for (int tm = 0; tm < ceil_div(b.n, sc_m); ++tm)
+            for (int tn = 0; tn < ceil_div(b.o + b.v, sc_n); ++tn) tsc.push_back(make_int4(I, 0, tm, tn));
         for (int s = 0; s < (fp64_products ? b.nr : 0); ++s) {
-            for (int tm = 0; tm < ceil_div(n2, GB_M); ++tm)
-                for (int tn = 0; tn < ceil_div(b.v, GB_N); ++tn) {
+            for (int tm = 0; tm < ceil_div(n2, BtTile::M); ++tm)
+                for (int tn = 0; tn < ceil_div(b.v, BtTile::N); ++tn) {
                     t1[g].push_back(make_int4(I, s, tm, tn));
-                    if (b.lc && !(b.nh && tm * GB_M >= b.n + b.nh)) t4[g].push_back(make_int4(I, s, tm, tn));
+                    if (b.lc && !(b.nh && tm * BtTile::M >= b.n + b.nh)) t4[g].push_back(make_int4(I, s, tm, tn));
                 }
             // with the block structure: F tiles that only hold zeros or values multiplied by zeros
             // are left out (as in the plane steps), G rows from n+nh are not needed
             if (b.lc)
-                for (int tm = 0; tm < ceil_div(n2, GB_M); ++tm)
-                    for (int tn = 0; tn < ceil_div(n2, GB_N); ++tn) {
-                        const int r0 = tm * GB_M, c0 = tn * GB_N;
-                        if (b.nh && !(bp_meets(r0, r0 + GB_M, 0, b.nh, b.n, b.n + b.nh) &&
-                                      bp_meets(c0, c0 + GB_N, b.nh, b.n, b.n + b.nh, n2)))
+                for (int tm = 0; tm < ceil_div(n2, BtTile::M); ++tm)
+                    for (int tn = 0; tn < ceil_div(n2, BtTile::N); ++tn) {
+                        const int r0 = tm * BtTile::M, c0 = tn * BtTile::N;
+                        if (b.nh && !(bp_meets(r0, r0 + BtTile::M, 0, b.nh, b.n, b.n + b.nh) &&
+                                      bp_meets(c0, c0 + BtTile::N, b.nh, b.n, b.n + b.nh, n2)))
                             continue;
                         t2[g].push_back(make_int4(I, s, tm, tn));
                     }
-            for (int tm = 0; tm < ceil_div(b.o, GB_M); ++tm)
-                for (int tn = 0; tn < ceil_div(b.v, GB_N); ++tn) t5[g].push_back(make_int4(I, s, tm, tn));
+            for (int tm = 0; tm < ceil_div(b.o, BtTile::M); ++tm)
+                for (int tn = 0; tn < ceil_div(b.v, BtTile::N); ++tn) t5[g].push_back(make_int4(I, s, tm, tn));
         }
     }
     upload_any(stream, w.t_sc, tsc);
