@@ -11,9 +11,11 @@ from tincr_gb300 import _lib
 from tincr_gb300 import tda as T
 
 # (orbitals, occupied, virtual, vectors): one tile and less, tile edges and one past them, odd sizes,
-# few vectors (small tiles) and many
+# few vectors (small FP64 tiles) and many; the last rows have enough work for the digit GEMMs (also in
+# more than one chunk of vectors)
 SIZES = [(4, 1, 3, 1), (16, 8, 8, 1), (17, 8, 9, 2), (33, 16, 17, 1), (48, 24, 24, 1), (65, 32, 33, 20), (96, 64, 32, 3),
-         (102, 51, 51, 5), (129, 64, 65, 2), (200, 99, 101, 7), (261, 130, 131, 1), (330, 200, 130, 11)]
+         (102, 51, 51, 5), (129, 64, 65, 2), (200, 99, 101, 7), (261, 130, 131, 1), (330, 200, 130, 11),
+         (17, 8, 9, 2200), (65, 32, 33, 70), (128, 64, 64, 12), (129, 64, 65, 12), (96, 31, 65, 20)]
 
 
 def _system(n, o, v, lc, seed):
@@ -63,3 +65,18 @@ def test_products_at_tile_edges(n, o, v, k, lc):
     terms = 2 * n + o + v + 2 * n + 2 * n + 2 * len(q["opa"]) + 20
     tol = terms * np.finfo(float).eps * _chain(q, n, o, v, x, True)
     assert np.all(np.abs(got - _chain(q, n, o, v, x, False)) <= tol)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,o,v,k", [(33, 16, 17, 2), (129, 64, 65, 12)])
+def test_products_scale_exactly(n, o, v, k):
+    """A power of two times X gives exactly that multiple of A.X, far from 1 too; zero gives zero."""
+    q = _system(n, o, v, True, n)
+    ctx = _lib.Context(0)
+    es = T.ExcitedStateSystem(ctx, q["opa"], q["c"], q["s"], q["orbe"], o, v, q["gamma"], q["glr"], q["xyz"])
+    x = np.random.default_rng(k).normal(size=(o * v, k))
+    x[:, 1] = 0.0
+    got = es.compute_products(x)
+    assert np.all(got[:, 1] == 0.0) and np.all(np.isfinite(got))
+    for p in (-400, 300):
+        assert np.array_equal(es.compute_products(np.ldexp(x, p)), np.ldexp(got, p))

@@ -115,14 +115,21 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
+// Output tiles of n_b products: 128 rows of A x 32 rows of B each, K split n_ks ways; product b's
+// operands start a_bt row tiles of A and b_bt of B after product b - 1's (0: shared), B at tile nt0.
+// Row tiles run fastest, so concurrent CTAs read the same B tile from L2.
 struct DgTiles {
-    int n_mt;   // 128-row tiles of A
-    int n_ks;   // K splits
-    int nkb;    // K blocks of 64
-    __device__ __forceinline__ int count() const { return n_mt * n_ks; }
-    __device__ __forceinline__ void decode(int t, int &mt, int &kb0, int &kb1) const {
+    int n_mt, n_nt, n_b, n_ks;
+    int nkb;   // K blocks of 64
+    int a_bt, b_bt, nt0;
+    __host__ __device__ __forceinline__ int count() const { return n_mt * n_nt * n_b * n_ks; }
+    __device__ __forceinline__ void decode(int t, int &mt, int &nt, int &b, int &kb0, int &kb1) const {
         mt = t % n_mt;
-        const int ks = t / n_mt;
+        t /= n_mt;
+        nt = t % n_nt;
+        t /= n_nt;
+        b = t % n_b;
+        const int ks = t / n_b;
         kb0 = (int)((long long)ks * nkb / n_ks);
         kb1 = (int)((long long)(ks + 1) * nkb / n_ks);
     }
@@ -131,7 +138,7 @@ struct DgTiles {
 template <class Epi>
 __global__ void __launch_bounds__(DG_T, 1)
 gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                   const __grid_constant__ CUtensorMap mapB4, DgTiles tl, int nbt, Epi epi, int *err) {
+                   const __grid_constant__ CUtensorMap mapB4, DgTiles tl, Epi epi, int *err) {
     extern __shared__ unsigned char dg_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)dg_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + 2 * DG_BUF);
@@ -168,8 +175,8 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
             int q = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-                int mt, kb0, kb1;
-                tl.decode(t, mt, kb0, kb1);
+                int mt, nt, pb, kb0, kb1;
+                tl.decode(t, mt, nt, pb, kb0, kb1);
                 for (int kb = kb0; kb < kb1 && ok; ++kb)
                     for (int h = 0; h < 2; ++h, ++q) {
                         const int s = q & 1;
@@ -181,8 +188,8 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                         unsigned char *st = smem + s * DG_BUF;
                         // the second half (A planes 4-7) pairs only with B planes 0-3
                         mbar_expect_tx(&full[s], 4 * DG_ATILE + (h ? 4 : DG_PLANES) * DG_BTILE);
-                        tma_load_5d(st, &mapA, kb, mt, 4 * h, &full[s]);
-                        tma_load_5d(st + 4 * DG_ATILE, h ? &mapB4 : &mapB, kb, nbt, 0, &full[s]);
+                        tma_load_5d(st, &mapA, kb, pb * tl.a_bt + mt, 4 * h, &full[s]);
+                        tma_load_5d(st + 4 * DG_ATILE, h ? &mapB4 : &mapB, kb, pb * tl.b_bt + tl.nt0 + nt, 0, &full[s]);
                     }
             }
             if (!ok)   // loads still in flight land before the CTA exits
@@ -193,8 +200,8 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
             int q = 0, c = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-                int mt, kb0, kb1;
-                tl.decode(t, mt, kb0, kb1);
+                int mt, nt, pb, kb0, kb1;
+                tl.decode(t, mt, nt, pb, kb0, kb1);
                 for (int kc = kb0; kc < kb1 && ok; kc += 2, ++c) {
                     const int a = c & 1;
                     if (c >= 2 && !mbar_wait(&acce[a], ((c >> 1) - 1) & 1)) {
@@ -246,8 +253,8 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
         int c = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-            int mt, kb0, kb1;
-            tl.decode(t, mt, kb0, kb1);
+            int mt, nt, pb, kb0, kb1;
+            tl.decode(t, mt, nt, pb, kb0, kb1);
             for (int kc = kb0; kc < kb1; kc += 2, ++c) {
                 const int a = c & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(&accf[a], (c >> 1) & 1));
@@ -268,11 +275,11 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        // exact integers below 2^24 in magnitude
-                        const long long v = ((((long long)__float2int_rz(__uint_as_float(r0[j])) << 7) +
+                        // exact integers of at most 2^24 in magnitude
+                        const long long v = ((((long long)__float2int_rz(__uint_as_float(r0[j])) << Epi::BITS) +
                                               (long long)__float2int_rz(__uint_as_float(r1[j])))
-                                                 << 14) +
-                                            ((long long)__float2int_rz(__uint_as_float(r2[j])) << 7) +
+                                                 << (2 * Epi::BITS)) +
+                                            ((long long)__float2int_rz(__uint_as_float(r2[j])) << Epi::BITS) +
                                             (long long)__float2int_rz(__uint_as_float(r3[j]));
                         if (lg == 0) H[j] += v;
                         else L[j] += v;
@@ -283,7 +290,7 @@ gemm_digits_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                 if (lane == 0) mbar_arrive(&acce[a]);
             }
             if (!ok) break;
-            if (kb1 > kb0) epi(mt * DG_M + quarter * 32 + lane, half * 16, H, L);
+            if (kb1 > kb0) epi(pb, mt * DG_M + quarter * 32 + lane, nt * DG_N + half * 16, H, L);
 #pragma unroll
             for (int j = 0; j < 16; ++j) H[j] = L[j] = 0;
         }
@@ -303,9 +310,10 @@ __device__ __forceinline__ double dg_value(long long H, long long L, double scal
 
 // split-K partial sums: exact int64 atomics into acc[(row * ldn + col) * 2 + {0, 1}] (rows < M, cols < N)
 struct DgEpiAtomic {
+    static constexpr int BITS = 7;   // bits of a digit
     unsigned long long *acc;
     int M, N, ldn;
-    __device__ __forceinline__ void operator()(int row, int col0, const long long (&H)[16],
+    __device__ __forceinline__ void operator()(int, int row, int col0, const long long (&H)[16],
                                                const long long (&L)[16]) const {
         if (row >= M) return;
 #pragma unroll
@@ -323,13 +331,14 @@ struct DgEpiAtomic {
 // linear combinations: value v of output (row = x, col = r) with scale[r] = 2^(Eb[r] - 63);
 // mode 0: out[r][x] = v;  1: out[r][x] = v - u[r] R[r][x] (residual);  2: out[r][x] -= v
 struct DgEpiComb {
+    static constexpr int BITS = 7;
     double *out;
     long long ld;
     const double *scale;
     int M, N, mode;
     const double *R;
     const double *u;
-    __device__ __forceinline__ void operator()(int row, int col0, const long long (&H)[16],
+    __device__ __forceinline__ void operator()(int, int row, int col0, const long long (&H)[16],
                                                const long long (&L)[16]) const {
         if (row >= M) return;
 #pragma unroll
@@ -363,15 +372,10 @@ inline CUtensorMap digit_map(const DgOperand &o, int box_planes) {
     return m;
 }
 
-// C tile loop over A rows [0, M) (128-row tiles) and the 32 B rows of row tile nbt, K = 64 nkb (at
-// most the operands' Kpad) split into n_ks ranges; persistent grid of at most n_sm CTAs.
+// One launch over the tiles tl of the digit operands A and B; persistent grid of at most n_sm CTAs.
 template <class Epi>
-void gemm_digits(cudaStream_t st, int n_sm, int M, int nkb, int n_ks, const DgOperand &A, const DgOperand &B, int nbt,
-                 Epi epi, int *d_err) {
-    if (M <= 0 || nkb <= 0) return;
-    if (A.rt_shift != 7 || B.rt_shift != 5 || (long long)nkb * DG_K > A.Kpad || (long long)nkb * DG_K > B.Kpad ||
-        M > A.rows_pad || (nbt + 1) * 32LL > B.rows_pad)
-        fail(TINCR_BAD_ARG, "gemm_digits: operand layout");
+void gemm_digits_tiles(cudaStream_t st, int n_sm, const DgTiles &tl, const DgOperand &A, const DgOperand &B, Epi epi,
+                       int *d_err) {
     const CUtensorMap ma = digit_map(A, 4);
     const CUtensorMap mb = digit_map(B, DG_PLANES);
     const CUtensorMap mb4 = digit_map(B, 4);
@@ -380,11 +384,22 @@ void gemm_digits(cudaStream_t st, int n_sm, int M, int nkb, int n_ks, const DgOp
         TINCR_CUDA(cudaFuncSetAttribute(gemm_digits_kernel<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
         attr = true;
     }
-    DgTiles tl{ceil_div(M, DG_M), std::max(1, std::min(n_ks, nkb)), nkb};
-    const int ntiles = tl.n_mt * tl.n_ks;
-    gemm_digits_kernel<Epi><<<std::min(ntiles, n_sm), DG_T, DG_SMEM, st>>>(ma, mb, mb4, tl, nbt, epi, d_err);
+    gemm_digits_kernel<Epi><<<std::min(tl.count(), n_sm), DG_T, DG_SMEM, st>>>(ma, mb, mb4, tl, epi, d_err);
     count_launch(st, "gemm_digits");
     check_launch("gemm_digits");
+}
+
+// C tile loop over A rows [0, M) (128-row tiles) and the 32 B rows of row tile nbt, K = 64 nkb (at
+// most the operands' Kpad) split into n_ks ranges.
+template <class Epi>
+void gemm_digits(cudaStream_t st, int n_sm, int M, int nkb, int n_ks, const DgOperand &A, const DgOperand &B, int nbt,
+                 Epi epi, int *d_err) {
+    if (M <= 0 || nkb <= 0) return;
+    if (A.rt_shift != 7 || B.rt_shift != 5 || (long long)nkb * DG_K > A.Kpad || (long long)nkb * DG_K > B.Kpad ||
+        M > A.rows_pad || (nbt + 1) * 32LL > B.rows_pad)
+        fail(TINCR_BAD_ARG, "gemm_digits: operand layout");
+    gemm_digits_tiles(st, n_sm, DgTiles{ceil_div(M, DG_M), 1, 1, std::max(1, std::min(n_ks, nkb)), nkb, 0, 0, nbt}, A, B,
+                      epi, d_err);
 }
 
 }  // namespace tincr

@@ -130,7 +130,7 @@ __global__ void diag_dots_kernel(int n, int v, const double *__restrict__ H, lon
 __global__ void __launch_bounds__(256)
 coulomb_kernel(int n, int n_atoms, const int *__restrict__ ao_off, const double *__restrict__ gamma,
                const double *__restrict__ d3, const double *__restrict__ d2, double *zao, double *F, double *y_out,
-               double scale) {
+               double scale, long long ldf, long long sbf, unsigned *fmx, int fmx_b) {
     extern __shared__ double sh[];
     double *y = sh;            // [n_atoms]
     const int b = blockIdx.y;
@@ -151,22 +151,30 @@ coulomb_kernel(int n, int n_atoms, const int *__restrict__ ao_off, const double 
     for (int B = lane; B < n_atoms; B += 32) z += g[B] * y[B];
     for (int off = 16; off; off >>= 1) z += __shfl_xor_sync(0xffffffffu, z, off);
     z *= scale;
-    const int n2 = 2 * n;
     for (int mu = ao_off[A] + lane; mu < ao_off[A + 1]; mu += 32) {
         if (zao) zao[(long long)b * n + mu] = z;
         if (F) {
-            double *f = F + (long long)b * n2 * n2;
-            f[(long long)mu * n2 + n + mu] += z;
-            f[(long long)(n + mu) * n2 + mu] += z;
+            double *f = F + (long long)b * sbf;
+            const double f01 = f[(long long)mu * ldf + n + mu] += z;
+            const double f10 = f[(long long)(n + mu) * ldf + mu] += z;
+            if (fmx) {
+                atomicMax(fmx + (long long)b * fmx_b + mu, (unsigned)__double2hiint(f01) & 0x7fffffffu);
+                atomicMax(fmx + (long long)b * fmx_b + n + mu, (unsigned)__double2hiint(f10) & 0x7fffffffu);
+            }
         }
     }
 }
 
 void launch_coulomb(cudaStream_t st, int kc, int n, int n_atoms, const int *ao_off, const double *gamma,
-                    const double *d3, const double *d2, double *zao, double *F, double *y_out, double scale) {
+                    const double *d3, const double *d2, double *zao, double *F, double *y_out, double scale,
+                    long long ldf, long long sbf, unsigned *fmx, int fmx_b) {
     dim3 g(ceil_div(n_atoms, COULOMB_ATOMS), kc);
+    if (ldf == 0) {
+        ldf = 2LL * n;
+        sbf = ldf * ldf;
+    }
     coulomb_kernel<<<g, 32 * COULOMB_ATOMS, n_atoms * sizeof(double), st>>>(n, n_atoms, ao_off, gamma, d3, d2, zao, F,
-                                                                            y_out, scale);
+                                                                            y_out, scale, ldf, sbf, fmx, fmx_b);
     count_launch(st, "coulomb");
     check_launch("coulomb");
 }
@@ -607,6 +615,7 @@ void Ctx::tda_setup(int n_atoms_, const int *opa, int n, const double *C, const 
     lc = gamma_lr != nullptr;
     upload_mo(n, C, S);
     planes_ready = false;
+    cd_ready = false;
     mx_key = -1;
     h_xyz.assign(xyz, xyz + 3 * (size_t)n_atoms);
     upload(stream, d_xyz, xyz, 3 * (size_t)n_atoms);
@@ -661,9 +670,13 @@ void Ctx::ao_contract(int k, int R, int S, const double *V, int P, int Q, double
         ao_contract_mixed(k, R, S, V, P, Q, ax, ac, out, alpha, beta, Xomega);
         return;
     }
+    const bool exch = ax != 0.0 && lc;
+    if ((exch || ac != 0.0) && digits_pay(k, R, S, P, Q, exch)) {
+        ao_contract_digits(k, R, S, V, P, Q, ax, ac, out, alpha, beta, Xomega);
+        return;
+    }
     const int n = n_orb;
     const int nr = bsz(R), ns = bsz(S), np = bsz(P), nq = bsz(Q);
-    const bool exch = ax != 0.0 && lc;
     const int kc_max = product_chunk();
     const int wmax = std::max(n_occ, n_virt);
     wsH.reserve((size_t)kc_max * 2 * n * wmax);

@@ -31,6 +31,14 @@ enum Blk { BLK_OCC = 0, BLK_VIRT = 1 };
 // tighter tolerances make a TINCR_PREC_BF16X3 solve finish with FP64 Davidson iterations.
 constexpr double MIXED_TOL_FLOOR = 1e-6;
 
+// FP64 multiply-adds above which the contraction runs as digit GEMMs (contract_digits.cu).  Below, the
+// twelve launches of that path (about 110 us in all) outweigh the FP64 pipe's 1.7 us per 1e6.  Device
+// time of a call, digits against FP64 tiles: decacene (n = 192) 1 vector, 35e6: 129 / 109 us;
+// pentacene (n = 102) 10 vectors, 53e6: 123 / 149; (H2O)48 (n = 288) 1 vector, 85e6: 148 / 190;
+// without exchange (H2O)64 1 vector, 50e6: 109 / 135.
+constexpr double CD_MIN_MAC = 45e6;
+
+struct DgOperand;                      // digit planes of a GEMM operand (digits.cuh)
 struct BatchWork;                      // batched LE / CT TDA workspace (batch.cu)
 void release_batch(BatchWork *w);
 // entries of the batch tile-shape autotuner's table (9 ints and 16 times each); returns the count
@@ -131,6 +139,20 @@ struct Ctx {
     void dg_ritz(int k, int m, const double *Yt, double *R, double *Rk, const double *u);
     void dg_ortho(int kadd, int m, double *T, double *cbuf);
     int dg_check();
+    // digit GEMMs of the FP64 contraction (contract_digits.cu): the system's orbital blocks, and the
+    // workspace of a chunk of vectors
+    bool cd_ready = false;
+    DevBuf<__nv_bfloat16> cd_blk[2], cd_pl;
+    DevBuf<int> cd_eblk[2], cd_int;
+    DevBuf<unsigned> cd_mx;
+    DevBuf<double> cd_f64;
+    DgOperand cd_stkA(int blk) const;     // [C_B;SC_B] in 128-row tiles
+    DgOperand cd_stkB(int blk) const;     // the same in 32-row tiles
+    DgOperand cd_swpT(int blk) const;     // [SC_B;C_B]^T in 32-row tiles
+    void prepare_digits();
+    bool digits_pay(int k, int R, int S, int P, int Q, bool exch) const;
+    void ao_contract_digits(int k, int R, int S, const double *V, int P, int Q, double ax, double ac, double *out,
+                            double alpha, double beta, const double *Xomega);
     void gemm_f64_digits(int M, int N, int K, const double *A, const double *B, double *C);
     BatchWork *batch = nullptr;
     PinnedBuf ex_pin;                     // staging of the exciton Hamiltonian's large inputs
