@@ -1,4 +1,5 @@
-// Batched SCC ground states (restricted closed shell, long-range corrected or not), one system per CTA.
+// Batched SCC ground states (restricted closed shell, long-range corrected or not), one system per
+// thread-block cluster.
 //
 // Follows tincr's SCC routine (src/scc/scc_routine.rs:121-290) together with the inputs it builds
 // first: overlap S and H0 from the Slater-Koster splines (src/scc/h0_and_s.rs:92-182), the Gaussian
@@ -9,30 +10,44 @@
 // Fock matrix (up to 8 iterates).  tincr mixes Mulliken charges with Broyden's method and stops at an
 // rms charge change of 1e-5: the same stationary density, reached here to a tighter test.
 //
-// Layout.  A persistent grid (two CTAs per SM) takes systems from a counter, largest first.  A CTA
-// keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and runs
-// every step itself:
+// Layout.  A persistent grid of clusters (two CTAs per SM) takes systems from a counter, largest first.
+// A cluster keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and
+// runs every step itself; its CTAs share out the tiles, rows, roots and elements of a step and meet at
+// the cluster barrier, small vectors and sums going straight into each other's shared memory:
 //  * GEMMs on tiles of 16 x 16 outputs, one per thread (FP64) or 32 x 32, 2 x 2 per thread (FP32).
 //    GB300 issues 2 FP64 FMAs per SM and clock against 128 FP32 FMAs, so the FP64 GEMMs are bound by
 //    the FP64 pipe and small tiles keep the padding of n = 48..256 matrices small;
-//  * eigenpairs: Householder tridiagonalisation, Sturm-count bisection with one thread per root,
-//    inverse iteration with one thread per root (LU with partial pivoting), Gram-Schmidt inside
-//    clusters of close roots (LAPACK dstein's criterion, 1e-3 of the tridiagonal's norm), and the
-//    back-transformation by the stored reflections;
-//  * the Fock build, Mulliken charges, DIIS and the energy as CTA-wide element loops and reductions.
+//  * eigenpairs: Householder tridiagonalisation, Sturm-count multisection (the lanes that the roots
+//    leave idle take more points per root), inverse iteration with one thread per root (LU with partial
+//    pivoting), Gram-Schmidt inside clusters of close roots (LAPACK dstein's criterion, 1e-3 of the
+//    tridiagonal's norm), and the back-transformation by the stored reflections;
+//  * the Fock build, Mulliken charges, DIIS and the energy as element loops and reductions.
+// CTAs per system: the largest power of two up to 16 that keeps the batch within SC_FILL CTAs per SM.
+// One CTA per system left most SMs idle on small batches and ended every batch with its slowest
+// system.  Measured, one CTA per system / the rule (ms of the kernel, LC, to 1e-10): one decacene
+// (192 orbitals, 16 CTAs) 705 / 123, 16 acene dimers (up to 186 orbitals) 690 / 160, 40 dimers 719 / 233,
+// 75 dimers 728 / 367, 128 dimers 750 / 417, 64 acenes 145 / 74, 400 dimers (1 CTA each) 1100 / 1081.
+// With 2 or 8 CTAs per SM instead of 4, 128 dimers take 600 / 561.  What bounds it: the FP64 pipe in the
+// GEMMs (40 % of a system's time at 4 CTAs), the FP64 latency chains of the eigensolver otherwise.
 // With TINCR_SCC_FP32_START the iterations run in FP32 until the commutator is below 1e-5 (at most
 // 60 of them), then continue in FP64 from that density with a fresh DIIS history: the stationary
 // point, the convergence test and the final orbitals are FP64 either way.
-// Every loop is bounded (max_iter, 80 bisection steps, 3 inverse iterations); there is no
-// inter-CTA waiting.  Non-finite values end the system's iterations and are reported.
+// Every loop is bounded (max_iter, 80 multisection steps, 3 inverse iterations); CTAs wait for each
+// other only at cluster barriers, which every thread of a cluster reaches the same number of times
+// (decisions come from values that every CTA forms from the same numbers in the same order).
+// Non-finite values end the system's iterations and are reported.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "sk_math.cuh"
 #include "tda.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tincr {
 
@@ -45,6 +60,9 @@ constexpr int SC_FP32_MAX = 20;        // FP32 iterations at most before the FP6
 constexpr double SC_FP32_SWITCH = 1e-5;
 constexpr double SC_PROXIMITY = 30.0;  // bohr: Slater-Koster pairs farther apart are zero (tincr's PROXIMITY_CUTOFF)
 constexpr int SC_SLOTS_PER_SM = 2;
+constexpr int SC_KS = 32;              // k depth of a GEMM slice
+constexpr int SC_CMAX = 16;            // CTAs per cluster
+constexpr int SC_FILL = 4;             // CTAs per SM that a batch is spread over (twice those that run at once)
 
 struct ScArgs {
     int n_sys;
@@ -70,13 +88,16 @@ struct ScArgs {
     // slots
     unsigned char *ws;
     long long slot_bytes, nn_max, at2_max, npad;
+    int csize;                         // CTAs per cluster (and system)
     int *next;
 };
 
-// shared memory of one CTA
+// shared memory of one CTA; arrays that every CTA of a cluster needs are held in each of them
 struct ScShared {
-    alignas(16) double gemm[2 * 16 * 17];               // GEMM tiles (FP64 16 x 17, FP32 16 x 33 each)
-    double d[SC_NMAX], e[SC_NMAX], beta[SC_NMAX], esq[SC_NMAX], vp[SC_NMAX], vu[SC_NMAX], vs[SC_NMAX];
+    alignas(16) double gemm[2 * SC_KS * 17];            // GEMM tiles (FP64 32 x 17, FP32 32 x 33 each); dot partials
+    double d[SC_NMAX], e[SC_NMAX], beta[SC_NMAX], esq[SC_NMAX], vu[SC_NMAX], cur[SC_NMAX];
+    double vp[2][SC_NMAX], rb[2][SC_NMAX];               // written by the other CTAs, alternating
+    double xch[2][SC_CMAX][SC_DIIS];                     // sums of every CTA, alternating
     double w[SC_NMAX];                                   // eigenvalues
     double qao[SC_NMAX], dq[SC_NMAX], esp[SC_NMAX];
     double red[SC_W * SC_DIIS + SC_DIIS + 8];
@@ -85,25 +106,65 @@ struct ScShared {
     double lin[(SC_DIIS + 1) * (SC_DIIS + 2)];
     int kind[SC_NMAX], ao_off[SC_NMAX + 1];
     short ao_atom[SC_NMAX];
-    int sys_id, flag;
+    int sys_id;
+    int rank, csize, par;   // CTA of the cluster, CTAs, parity of the next exchange
 };
 
-// ---------------------------------------------------------------------------------------------
-// CTA-wide reductions (every thread receives the result)
-// ---------------------------------------------------------------------------------------------
+// The CTAs of a cluster work on one system.  SC_FOR: an element loop over all their threads;
+// sc_bar: what they wrote to global (and to each other's shared) memory is visible after it.
+#define SC_FOR(t, count) \
+    for (long long t = (long long)sm.rank * SC_T + threadIdx.x; t < (count); t += (long long)sm.csize * SC_T)
 
-__device__ double sc_sum(double v, ScShared &sm) {
-    for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
-    for (int w = 0; w < SC_W; ++w) s += sm.red[w];
-    __syncthreads();
-    return s;
+__device__ __forceinline__ void sc_bar(const ScShared &sm) {
+    if (sm.csize > 1) cg::this_cluster().sync();
+    else __syncthreads();
 }
 
-__device__ double sc_max(double v, ScShared &sm) {
+// the same variable in CTA r of the cluster
+template <class V>
+__device__ __forceinline__ V *sc_at(V *x, int r) { return cg::this_cluster().map_shared_rank(x, r); }
+
+// ---------------------------------------------------------------------------------------------
+// Reductions (every thread of every CTA receives the result)
+// ---------------------------------------------------------------------------------------------
+
+// m sums (m <= SC_DIIS) of the CTA into sm.red[SC_W * SC_DIIS + r], then over the cluster in CTA order
+__device__ void sc_sums(double *v, int m, ScShared &sm) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+    for (int r = 0; r < m; ++r) {
+        double x = v[r];
+        for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+        if (lane == 0) sm.red[warp * SC_DIIS + r] = x;
+    }
+    __syncthreads();
+    const int par = sm.par;
+    if (threadIdx.x < m) {
+        double s = 0.0;
+        for (int w = 0; w < SC_W; ++w) s += sm.red[w * SC_DIIS + threadIdx.x];
+        sm.red[SC_W * SC_DIIS + threadIdx.x] = s;
+        if (sm.csize > 1)
+            for (int c = 0; c < sm.csize; ++c) *sc_at(&sm.xch[par][sm.rank][threadIdx.x], c) = s;
+    }
+    if (sm.csize > 1) {
+        sc_bar(sm);   // a CTA writes this parity again only after the next exchange's barrier
+        if (threadIdx.x < m) {
+            double s = 0.0;
+            for (int c = 0; c < sm.csize; ++c) s += sm.xch[par][c][threadIdx.x];
+            sm.red[SC_W * SC_DIIS + threadIdx.x] = s;
+        }
+        if (threadIdx.x == 0) sm.par = par ^ 1;
+    }
+    __syncthreads();
+}
+
+__device__ double sc_sum(double v, ScShared &sm) {
+    sc_sums(&v, 1, sm);
+    return sm.red[SC_W * SC_DIIS];
+}
+
+// maximum over the CTA
+__device__ double sc_max_cta(double v, ScShared &sm) {
     for (int off = 16; off; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
@@ -114,70 +175,74 @@ __device__ double sc_max(double v, ScShared &sm) {
     return s;
 }
 
-// m sums (m <= SC_DIIS) at once; out in sm.red[SC_W * SC_DIIS + r]
-__device__ void sc_sums(double *v, int m, ScShared &sm) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = 0; r < m; ++r) {
-        double x = v[r];
-        for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-        if (lane == 0) sm.red[warp * SC_DIIS + r] = x;
+// maximum over the cluster
+__device__ double sc_max(double v, ScShared &sm) {
+    double s = sc_max_cta(v, sm);
+    if (sm.csize > 1) {
+        const int par = sm.par;
+        if (threadIdx.x < sm.csize) *sc_at(&sm.xch[par][sm.rank][0], (int)threadIdx.x) = s;
+        sc_bar(sm);
+        for (int c = 0; c < sm.csize; ++c) s = fmax(s, sm.xch[par][c][0]);
+        __syncthreads();
+        if (threadIdx.x == 0) sm.par = par ^ 1;
+        __syncthreads();
     }
-    __syncthreads();
-    if (threadIdx.x < m) {
-        double s = 0.0;
-        for (int w = 0; w < SC_W; ++w) s += sm.red[w * SC_DIIS + threadIdx.x];
-        sm.red[SC_W * SC_DIIS + threadIdx.x] = s;
-    }
-    __syncthreads();
+    return s;
 }
 
 // ---------------------------------------------------------------------------------------------
-// CTA GEMM: C = alpha op(A) op(B) + beta C, row-major, op(A) M x K, op(B) K x N (beta = 0: C not read).
+// GEMM of the cluster: C = alpha op(A) op(B) + beta C, row-major, op(A) M x K, op(B) K x N (beta = 0: C
+// not read); the tiles are dealt to the CTAs.
 // Tiles of TL = 16 R outputs square; thread (ty, tx) computes rows R ty + i, columns R tx + j.
 // ---------------------------------------------------------------------------------------------
 
 template <class T, int R>
 __device__ void sc_gemm(int M, int N, int K, T alpha, const T *A, int lda, bool ta, const T *B, int ldb, bool tb,
                         T beta, T *C, int ldc, ScShared &sm, bool sym) {
-    constexpr int TL = 16 * R;
+    constexpr int TL = 16 * R, PE = TL * SC_KS / SC_T;
     T(*As)[TL + 1] = reinterpret_cast<T(*)[TL + 1]>(sm.gemm);
-    T(*Bs)[TL + 1] = reinterpret_cast<T(*)[TL + 1]>(reinterpret_cast<T *>(sm.gemm) + 16 * (TL + 1));
+    T(*Bs)[TL + 1] = reinterpret_cast<T(*)[TL + 1]>(reinterpret_cast<T *>(sm.gemm) + SC_KS * (TL + 1));
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     const int tm = (M + TL - 1) / TL, tn = (N + TL - 1) / TL;
-    for (int t = 0; t < tm * tn; ++t) {
-        if (sym && t / tn < t % tn) continue;   // symmetric result: tiles on and below the diagonal only
-        const int m0 = (t / tn) * TL, n0 = (t % tn) * TL;
+    // symmetric result: the tiles on and below the diagonal, row by row
+    const int count = sym ? tm * (tm + 1) / 2 : tm * tn;
+    for (int t = sm.rank; t < count; t += sm.csize) {
+        int ti = t / tn, tj = t % tn;
+        if (sym) {
+            ti = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+            while (ti * (ti + 1) / 2 > t) --ti;
+            while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+            tj = t - ti * (ti + 1) / 2;
+        }
+        const int m0 = ti * TL, n0 = tj * TL;
         T acc[R][R];
 #pragma unroll
         for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int j = 0; j < R; ++j) acc[i][j] = T(0);
-        for (int k0 = 0; k0 < K; k0 += 16) {
+        T ra[PE], rb[PE];
+        auto load = [&](int k0) {
 #pragma unroll
-            for (int q = 0; q < R; ++q) {
-                const int e = tid + q * SC_T;   // 0 .. 16 TL - 1
-                if (!ta) {
-                    const int mm = e >> 4, kk = e & 15;
-                    const int m = m0 + mm, k = k0 + kk;
-                    As[kk][mm] = (m < M && k < K) ? A[(long long)m * lda + k] : T(0);
-                } else {
-                    const int kk = e / TL, mm = e % TL;
-                    const int m = m0 + mm, k = k0 + kk;
-                    As[kk][mm] = (m < M && k < K) ? A[(long long)k * lda + m] : T(0);
-                }
-                if (!tb) {
-                    const int kk = e / TL, nn = e % TL;
-                    const int n = n0 + nn, k = k0 + kk;
-                    Bs[kk][nn] = (n < N && k < K) ? B[(long long)k * ldb + n] : T(0);
-                } else {
-                    const int nn = e >> 4, kk = e & 15;
-                    const int n = n0 + nn, k = k0 + kk;
-                    Bs[kk][nn] = (n < N && k < K) ? B[(long long)n * ldb + k] : T(0);
-                }
+            for (int q = 0; q < PE; ++q) {
+                const int e = tid + q * SC_T;   // 0 .. SC_KS TL - 1
+                const int m = m0 + (ta ? e % TL : e / SC_KS), ka = k0 + (ta ? e / TL : e % SC_KS);
+                ra[q] = (m < M && ka < K) ? (ta ? A[(long long)ka * lda + m] : A[(long long)m * lda + ka]) : T(0);
+                const int n = n0 + (tb ? e / SC_KS : e % TL), kb = k0 + (tb ? e % SC_KS : e / TL);
+                rb[q] = (n < N && kb < K) ? (tb ? B[(long long)n * ldb + kb] : B[(long long)kb * ldb + n]) : T(0);
             }
+        };
+        load(0);
+        for (int k0 = 0; k0 < K; k0 += SC_KS) {
             __syncthreads();
 #pragma unroll
-            for (int kk = 0; kk < 16; ++kk) {
+            for (int q = 0; q < PE; ++q) {
+                const int e = tid + q * SC_T;
+                As[ta ? e / TL : e % SC_KS][ta ? e % TL : e / SC_KS] = ra[q];
+                Bs[tb ? e % SC_KS : e / TL][tb ? e / SC_KS : e % TL] = rb[q];
+            }
+            __syncthreads();
+            if (k0 + SC_KS < K) load(k0 + SC_KS);
+            auto step = [&](int kk) {
                 T a[R], b[R];
 #pragma unroll
                 for (int i = 0; i < R; ++i) a[i] = As[kk][R * ty + i];
@@ -187,28 +252,28 @@ __device__ void sc_gemm(int M, int N, int K, T alpha, const T *A, int lda, bool 
                 for (int i = 0; i < R; ++i)
 #pragma unroll
                     for (int j = 0; j < R; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            };
+            if (K - k0 >= SC_KS) {
+#pragma unroll
+                for (int kk = 0; kk < SC_KS; ++kk) step(kk);
+            } else {
+                for (int kk = 0; kk < K - k0; ++kk) step(kk);
             }
-            __syncthreads();
         }
 #pragma unroll
         for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 const int m = m0 + R * ty + i, n = n0 + R * tx + j;
-                if (m < M && n < N) {
+                if (m < M && n < N && !(sym && n > m)) {
                     T *c = C + (long long)m * ldc + n;
-                    *c = beta == T(0) ? alpha * acc[i][j] : fma(alpha, acc[i][j], beta * *c);
+                    const T v = beta == T(0) ? alpha * acc[i][j] : fma(alpha, acc[i][j], beta * *c);
+                    *c = v;
+                    if (sym && n < m) C[(long long)n * ldc + m] = v;
                 }
             }
     }
-    __syncthreads();
-    if (sym) {   // upper triangle from the lower one (C and, with beta != 0, its old value symmetric)
-        for (long long e = tid; e < (long long)M * M; e += SC_T) {
-            const int i = (int)(e / M), j = (int)(e - (long long)i * M);
-            if (i < j) C[(long long)i * ldc + j] = C[(long long)j * ldc + i];
-        }
-        __syncthreads();
-    }
+    sc_bar(sm);
 }
 
 template <class T> struct ScTile;
@@ -297,55 +362,77 @@ __device__ __forceinline__ int sc_sturm(const float *d, const float *esq, int n,
 // k-th Householder vector in columns k+1..n-1).  Eigenvalues ascending into sm.w (as double),
 // eigenvectors into Z [n x nr] row-major (column r = eigenvector r).  ws: 4 n nr elements, piv: n nr
 // bytes.  Returns false on a non-finite value.
+// CTA c of the cluster owns the rows i with i % csize = c of A in the tridiagonalisation and a
+// contiguous range of the roots afterwards.  The tridiagonalisation passes one cluster barrier per
+// column: before it every CTA sends its elements of p to the others' shared memory and the owner of the
+// next pivot row sends that row; after it each forms the updated pivot row (and so the next
+// reflection) itself.
 template <class T>
 __device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, ScShared &sm) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cs = sm.csize, rank = sm.rank;
     T *d = reinterpret_cast<T *>(sm.d), *e = reinterpret_cast<T *>(sm.e), *beta = reinterpret_cast<T *>(sm.beta);
-    T *esq = reinterpret_cast<T *>(sm.esq), *p = reinterpret_cast<T *>(sm.vp), *u = reinterpret_cast<T *>(sm.vu);
-    T *s = reinterpret_cast<T *>(sm.vs);
-    // 1. tridiagonalisation: H_k = I - beta_k u u^T acting on rows / columns k+1..n-1
+    T *esq = reinterpret_cast<T *>(sm.esq), *u = reinterpret_cast<T *>(sm.vu), *cur = reinterpret_cast<T *>(sm.cur);
+    // 1. tridiagonalisation: H_k = I - beta_k u u^T acting on rows / columns k+1..n-1; cur = row k of
+    //    the reduced matrix from column k
+    for (int i = tid; i < n; i += SC_T) cur[i] = A[i];
+    __syncthreads();
     for (int k = 0; k + 2 < n; ++k) {
         const int n1 = n - k - 1;
-        T *row = A + (long long)k * n + (k + 1);
+        T *p = reinterpret_cast<T *>(sm.vp[k & 1]), *nxt = reinterpret_cast<T *>(sm.rb[k & 1]);
         if (warp == 0) {
             T s2 = T(0);
-            for (int i = 1 + lane; i < n1; i += 32) s2 += row[i] * row[i];
+            for (int i = 1 + lane; i < n1; i += 32) s2 += cur[1 + i] * cur[1 + i];
             for (int off = 16; off; off >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-            const T x0 = row[0];
+            const T x0 = cur[1];
             T bet = T(0), alpha = x0;
             if (s2 != T(0)) {
                 const T nx = sqrt(x0 * x0 + s2);
                 alpha = x0 > T(0) ? -nx : nx;
                 bet = T(1) / (alpha * (alpha - x0));
             }
-            for (int i = 1 + lane; i < n1; i += 32) u[i] = row[i];
+            for (int i = 1 + lane; i < n1; i += 32) u[i] = cur[1 + i];
             if (lane == 0) {
-                d[k] = A[(long long)k * n + k];
+                d[k] = cur[0];
                 e[k] = alpha;
                 beta[k] = bet;
                 u[0] = x0 - alpha;
-                row[0] = x0 - alpha;
             }
         }
         __syncthreads();
         const T bet = beta[k];
-        if (bet == T(0)) continue;   // the same in every thread
+        if (k % cs == rank)
+            for (int i = tid; i < n1; i += SC_T) A[(long long)k * n + (k + 1 + i)] = u[i];
+        if ((k + 1) % cs == rank)
+            for (int i = tid; i < n1; i += SC_T) {
+                const T v = A[(long long)(k + 1) * n + (k + 1 + i)];
+                if (cs == 1) nxt[i] = v;
+                else
+                    for (int c = 0; c < cs; ++c) *sc_at(nxt + i, c) = v;
+            }
+        // own rows of the reduced matrix: first, first + cs, ...
+        const int first = (rank - (k + 1) % cs + cs) % cs, own = first < n1 ? (n1 - 1 - first) / cs + 1 : 0;
         {   // p = bet A' u, G lanes per row
             const int G = n1 >= 64 ? 32 : (n1 >= 16 ? 8 : 2);
             const int rows_per_pass = SC_T / G;
             const int sub = tid % G;
-            for (int base = 0; base < n1; base += rows_per_pass) {   // the same trip count in every thread
-                const int r0 = base + tid / G;
+            for (int base = 0; base < own; base += rows_per_pass) {   // the same trip count in every thread
+                const int q = base + tid / G, r0 = first + q * cs;
                 T acc = T(0);
-                if (r0 < n1) {
+                if (q < own) {
                     const T *ar = A + (long long)(k + 1 + r0) * n + (k + 1);
                     for (int j = sub; j < n1; j += G) acc = fma(ar[j], u[j], acc);
                 }
                 for (int off = G >> 1; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-                if (sub == 0 && r0 < n1) p[r0] = bet * acc;
+                if (q < own) {
+                    if (cs == 1) {
+                        if (sub == 0) p[r0] = bet * acc;
+                    } else {
+                        for (int c = sub; c < cs; c += G) *sc_at(p + r0, c) = bet * acc;
+                    }
+                }
             }
         }
-        __syncthreads();
+        sc_bar(sm);
         if (warp == 0) {   // q = p - (bet u.p / 2) u
             T up = T(0);
             for (int i = lane; i < n1; i += 32) up += u[i] * p[i];
@@ -354,19 +441,19 @@ __device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, Sc
             for (int i = lane; i < n1; i += 32) p[i] -= K * u[i];
         }
         __syncthreads();
-        for (int t = tid; t < n1 * n1; t += SC_T) {   // A' -= u q^T + q u^T
-            const int i = t / n1, j = t - i * n1;
+        for (int t = tid; t < own * n1; t += SC_T) {   // A' -= u q^T + q u^T
+            const int q = t / n1, i = first + q * cs, j = t - q * n1;
             T *a = A + (long long)(k + 1 + i) * n + (k + 1 + j);
             *a = fma(-u[i], p[j], fma(-p[i], u[j], *a));
         }
+        for (int j = tid; j < n1; j += SC_T) cur[j] = fma(-u[0], p[j], fma(-p[0], u[j], nxt[j]));
         __syncthreads();
     }
+    sc_bar(sm);   // the last row and every Householder vector
     if (tid == 0) {
-        if (n >= 2) {
-            d[n - 2] = A[(long long)(n - 2) * n + n - 2];
-            e[n - 2] = A[(long long)(n - 2) * n + n - 1];
-            beta[n - 2] = T(0);
-        }
+        d[n - 2] = cur[0];
+        e[n - 2] = cur[1];
+        beta[n - 2] = T(0);
         d[n - 1] = A[(long long)(n - 1) * n + n - 1];
         e[n - 1] = T(0);
         beta[n - 1] = T(0);
@@ -383,29 +470,54 @@ __device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, Sc
         emax2 = fmax(emax2, (double)esq[i]);
         fin = fin && isfinite((double)d[i]) && isfinite((double)e[i]);
     }
-    glo = -sc_max(-glo, sm);
-    ghi = sc_max(ghi, sm);
-    emax2 = sc_max(emax2, sm);
-    if (sc_max(fin ? 0.0 : 1.0, sm) != 0.0) return false;
+    glo = -sc_max_cta(-glo, sm);
+    ghi = sc_max_cta(ghi, sm);
+    emax2 = sc_max_cta(emax2, sm);
+    if (sc_max_cta(fin ? 0.0 : 1.0, sm) != 0.0) return false;   // the same in every CTA
     const double eps = ScEps<T>::eps;
     const double tnorm = fmax(fabs(glo), fabs(ghi));
     const double pivmin = ScEps<T>::tiny * fmax(1.0, emax2) * 4.0;
-    // 3. eigenvalue r by bisection on Sturm counts, one thread per root
-    for (int r = tid; r < nr; r += SC_T) {
+    const int chunk = (nr + cs - 1) / cs, rbeg = min(rank * chunk, nr), nc = min(chunk, nr - rbeg);   // own roots
+    // 3. eigenvalues by multisection on Sturm counts: P lanes per root take P points of its interval
+    //    (an FP64 warp instruction costs the same for one lane as for 32), as many as keep one warp per
+    //    sub-partition; P = 1 is bisection with one thread per root
+    int P = 1;
+    while (P < 32 && 2 * P * chunk <= 128) P *= 2;
+    for (int base = 0; base < nc * P; base += SC_T) {   // the same trip count in every thread
+        const int id = base + tid, r = rbeg + id / P, j = id % P;
+        bool active = id < nc * P;
+        const unsigned group = (P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1)));
         T a = (T)(glo - (2.0 * eps * tnorm + 2.0 * pivmin)), b = (T)(ghi + (2.0 * eps * tnorm + 2.0 * pivmin));
-        for (int it = 0; it < 80; ++it) {
-            const T mid = T(0.5) * (a + b);
-            if (!(b - a > T(2.0 * eps) * fmax(fabs(a), fabs(b)) + T(pivmin)) || mid <= a || mid >= b) break;
-            if (sc_sturm(d, esq, n, mid) > r) b = mid; else a = mid;
+        for (int it = 0; it < 80 && __any_sync(0xffffffffu, active); ++it) {
+            const T mag = fmax(fabs(a), fabs(b));
+            // bisection near the end, where the points would fall on neighbouring numbers
+            const bool bis = P == 1 || !(b - a > T(64.0 * eps) * mag);
+            const T h = (b - a) / T(P + 1);
+            auto point = [&](int i) { return bis ? T(0.5) * (a + b) : a + T(i + 1) * h; };
+            const T x = point(j);
+            if (!(b - a > T(2.0 * eps) * mag + T(pivmin)) || x <= a || x >= b) active = false;
+            const bool above = active && sc_sturm(d, esq, n, x) > r;
+            const unsigned m = (__ballot_sync(0xffffffffu, above) & group) >> (lane & ~(P - 1));
+            if (active) {
+                const int f = m ? __ffs(m) - 1 : P;   // first point above the root
+                const T na = f > 0 ? point(f - 1) : a, nb = f < P ? point(f) : b;
+                a = na;
+                b = nb;
+            }
         }
-        sm.w[r] = 0.5 * ((double)a + (double)b);
+        if (id < nc * P && j == 0) {
+            const double w = 0.5 * ((double)a + (double)b);
+            if (cs == 1) sm.w[r] = w;
+            else
+                for (int c = 0; c < cs; ++c) *sc_at(&sm.w[r], c) = w;
+        }
     }
-    __syncthreads();
+    sc_bar(sm);
     // 4. inverse iteration, one thread per root: LU of T - w_r I with partial pivoting (factors
     //    interleaved over the roots, [i * nr + r], so a warp's accesses are contiguous), then three
     //    solves from a fixed start vector; the recurrences run in registers
     const T tiny = (T)(eps * fmax(tnorm, 1e-30));
-    for (int r = tid; r < nr; r += SC_T) {
+    for (int r = rbeg + tid; r < rbeg + nc; r += SC_T) {
         const T lam = (T)sm.w[r];
         T *__restrict__ DL = ws;
         T *__restrict__ DD = ws + (long long)n * nr;
@@ -471,52 +583,125 @@ __device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, Sc
         }
 #undef IX
     }
-    __syncthreads();
-    // 5. Gram-Schmidt (twice) inside clusters of roots closer than 1e-3 |T| (warp 0, ascending)
-    if (warp == 0) {
+    sc_bar(sm);
+    // 5. Gram-Schmidt (twice) inside clusters of roots closer than 1e-3 |T|, one warp per cluster
+    {
         const double ortol = 1e-3 * tnorm;
-        int c0 = 0;
+        int c0 = 0, id = 0;
         for (int r = 1; r < nr; ++r) {
             if (sm.w[r] - sm.w[r - 1] > ortol) {
                 c0 = r;
+                ++id;
                 continue;
             }
+            if (id % (SC_W * cs) != rank * SC_W + warp) continue;
+            // root r in registers, row lane + 32 q in z[q]; its predecessors stream through
+            T z[SC_NMAX / 32], y[SC_NMAX / 32];
+            auto read = [&](int root, T (&x)[SC_NMAX / 32]) {
+#pragma unroll
+                for (int q = 0; q < SC_NMAX / 32; ++q)
+                    x[q] = lane + 32 * q < n ? Z[(long long)(lane + 32 * q) * nr + root] : T(0);
+            };
+            read(r, z);
             for (int pass = 0; pass < 2; ++pass)
-                for (int q = c0; q < r; ++q) {
+                for (int p = c0; p < r; ++p) {
+                    read(p, y);
                     T dot = T(0);
-                    for (int i = lane; i < n; i += 32) dot += Z[(long long)i * nr + q] * Z[(long long)i * nr + r];
+#pragma unroll
+                    for (int q = 0; q < SC_NMAX / 32; ++q)
+                        if (32 * q < n) dot = fma(y[q], z[q], dot);
                     for (int off = 16; off; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
-                    for (int i = lane; i < n; i += 32) Z[(long long)i * nr + r] -= dot * Z[(long long)i * nr + q];
-                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < SC_NMAX / 32; ++q)
+                        if (32 * q < n) z[q] = fma(-dot, y[q], z[q]);
                 }
             T nrm = T(0);
-            for (int i = lane; i < n; i += 32) nrm += Z[(long long)i * nr + r] * Z[(long long)i * nr + r];
+#pragma unroll
+            for (int q = 0; q < SC_NMAX / 32; ++q)
+                if (32 * q < n) nrm = fma(z[q], z[q], nrm);
             for (int off = 16; off; off >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, off);
             nrm = T(1) / sqrt(nrm);
-            for (int i = lane; i < n; i += 32) Z[(long long)i * nr + r] *= nrm;
-            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < SC_NMAX / 32; ++q)
+                if (lane + 32 * q < n) Z[(long long)(lane + 32 * q) * nr + r] = z[q] * nrm;
         }
     }
-    __syncthreads();
-    // 6. back-transformation Z <- H_0 ... H_{n-3} Z
-    for (int k = n - 3; k >= 0; --k) {
-        const T bet = beta[k];
-        if (bet == T(0)) continue;
-        const int n1 = n - k - 1;
-        const T *uk = A + (long long)k * n + (k + 1);
-        for (int r = tid; r < nr; r += SC_T) {
+    sc_bar(sm);
+    // 6. back-transformation Z <- H_0 ... H_{n-3} Z of the own columns (no exchange between CTAs)
+    if (chunk <= 2 * SC_W) {
+        // few columns: two per warp in registers, row lane + 32 q in z[q]
+        const int r0 = rbeg + warp, r1 = r0 + SC_W;
+        const bool h0 = warp < nc, h1 = warp + SC_W < nc;
+        T z0[SC_NMAX / 32], z1[SC_NMAX / 32];
+#pragma unroll
+        for (int q = 0; q < SC_NMAX / 32; ++q) {
+            const int i = lane + 32 * q;
+            z0[q] = h0 && i < n ? Z[(long long)i * nr + r0] : T(0);
+            z1[q] = h1 && i < n ? Z[(long long)i * nr + r1] : T(0);
+        }
+        if (h0)
+            for (int k = n - 3; k >= 0; --k) {
+                const T bet = beta[k];
+                if (bet == T(0)) continue;
+                T uk[SC_NMAX / 32], s0 = T(0), s1 = T(0);
+#pragma unroll
+                for (int q = 0; q < SC_NMAX / 32; ++q) {
+                    const int i = lane + 32 * q;
+                    if (32 * q + 31 <= k || 32 * q >= n) continue;   // the same in every lane
+                    uk[q] = i > k && i < n ? A[(long long)k * n + i] : T(0);
+                    s0 = fma(uk[q], z0[q], s0);
+                    if (h1) s1 = fma(uk[q], z1[q], s1);
+                }
+                for (int off = 16; off; off >>= 1) {
+                    s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+                    if (h1) s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+                }
+                s0 *= -bet;
+                s1 *= -bet;
+#pragma unroll
+                for (int q = 0; q < SC_NMAX / 32; ++q) {
+                    if (32 * q + 31 <= k || 32 * q >= n) continue;
+                    z0[q] = fma(s0, uk[q], z0[q]);
+                    if (h1) z1[q] = fma(s1, uk[q], z1[q]);
+                }
+            }
+#pragma unroll
+        for (int q = 0; q < SC_NMAX / 32; ++q) {
+            const int i = lane + 32 * q;
+            if (h0 && i < n) Z[(long long)i * nr + r0] = z0[q];
+            if (h1 && i < n) Z[(long long)i * nr + r1] = z1[q];
+        }
+    } else {
+        // `sub` threads per column, each with the rows i = sb (mod sub); the dots' parts alternate
+        // between two buffers, so one barrier per reflection
+        const int ncp = (nc + 31) / 32 * 32, sub = ncp > 0 ? SC_T / ncp : 1, c = ncp > 0 ? tid % ncp : 0;
+        const int sb = ncp > 0 ? tid / ncp : 0;
+        const bool on = c < nc && sb < sub;
+        T *Zc = Z + rbeg + c;
+        int buf = 0;
+        for (int k = n - 3; k >= 0; --k) {
+            const T bet = beta[k];
+            if (bet == T(0)) continue;
+            T *part = reinterpret_cast<T *>(sm.gemm) + buf * SC_T;
+            buf ^= 1;
+            const T *uk = A + (long long)k * n;
+            const int i0 = k + 1 + ((sb - (k + 1)) % sub + sub) % sub;
             T acc = T(0);
-            for (int i = 0; i < n1; ++i) acc = fma(uk[i], Z[(long long)(k + 1 + i) * nr + r], acc);
-            s[r] = bet * acc;
+            if (on)
+#pragma unroll 4
+                for (int i = i0; i < n; i += sub) acc = fma(uk[i], Zc[(long long)i * nr], acc);
+            part[tid] = acc;
+            __syncthreads();
+            if (on) {
+                T v = T(0);
+                for (int q = 0; q < sub; ++q) v += part[q * ncp + c];
+                v *= -bet;
+#pragma unroll 4
+                for (int i = i0; i < n; i += sub) Zc[(long long)i * nr] = fma(v, uk[i], Zc[(long long)i * nr]);
+            }
         }
-        __syncthreads();
-        for (int t = tid; t < n1 * nr; t += SC_T) {
-            const int i = t / nr, r = t - i * nr;
-            T *z = Z + (long long)(k + 1 + i) * nr + r;
-            *z = fma(-s[r], uk[i], *z);
-        }
-        __syncthreads();
     }
+    sc_bar(sm);
     return true;
 }
 
@@ -593,7 +778,7 @@ __device__ double sc_setup(const ScArgs &a, const tincr_scc_system &sy, const Sc
         for (int mu = sm.ao_off[A]; mu < sm.ao_off[A + 1]; ++mu) sm.ao_atom[mu] = (short)A;
     __syncthreads();
     const long long nn = (long long)n * n;
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         double sv = 0.0, hv = 0.0;
         if (mu == nu) {
@@ -604,12 +789,12 @@ __device__ double sc_setup(const ScArgs &a, const tincr_scc_system &sy, const Sc
         sl.S[t] = a.s_in ? a.s_in[sy.mat_off + t] : sv;
         sl.H0[t] = a.h0_in ? a.h0_in[sy.mat_off + t] : hv;
     }
-    __syncthreads();
+    sc_bar(sm);
     const bool build_sk = !a.s_in || !a.h0_in;
     // atom pairs A < B
     double erep = 0.0;
-    for (int t = tid; t < N * N; t += SC_T) {
-        const int A = t / N, B = t - A * N;
+    SC_FOR(t, N * N) {
+        const int A = (int)(t / N), B = (int)(t - (long long)A * N);
         const int kA = sm.kind[A], kB = sm.kind[B];
         const double dx = xyz[3 * B] - xyz[3 * A], dy = xyz[3 * B + 1] - xyz[3 * A + 1], dz = xyz[3 * B + 2] - xyz[3 * A + 2];
         const double r = sqrt(dx * dx + dy * dy + dz * dz);
@@ -675,7 +860,8 @@ __device__ double sc_setup(const ScArgs &a, const tincr_scc_system &sy, const Sc
                 }
             }
     }
-    const double e = sc_sum(erep, sm);   // synchronises
+    const double e = sc_sum(erep, sm);
+    sc_bar(sm);
     return e;
 }
 
@@ -687,14 +873,19 @@ __device__ double sc_setup(const ScArgs &a, const tincr_scc_system &sy, const Sc
 template <class T>
 __device__ void sc_charges(int n, int N, const T *P, const T *S, const T *gam, const double *p0, ScShared &sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int mu = warp; mu < n; mu += SC_W) {
+    for (int mu = sm.rank * SC_W + warp; mu < n; mu += SC_W * sm.csize) {
         T acc = T(0);
         const T *pr = P + (long long)mu * n, *sr = S + (long long)mu * n;
         for (int nu = lane; nu < n; nu += 32) acc = fma(pr[nu], sr[nu], acc);
         for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        if (lane == 0) sm.qao[mu] = (double)acc - p0[mu];   // S_mumu = 1
+        const double q = (double)acc - p0[mu];   // S_mumu = 1
+        if (sm.csize == 1) {
+            if (lane == 0) sm.qao[mu] = q;
+        } else if (lane < sm.csize) {
+            *sc_at(&sm.qao[mu], lane) = q;
+        }
     }
-    __syncthreads();
+    sc_bar(sm);
     for (int A = tid; A < N; A += SC_T) {
         double q = 0.0;
         for (int mu = sm.ao_off[A]; mu < sm.ao_off[A + 1]; ++mu) q += sm.qao[mu];
@@ -712,47 +903,46 @@ __device__ void sc_charges(int n, int N, const T *P, const T *S, const T *gam, c
 // F = H0 + 1/2 S o (esp_mu + esp_nu) [+ H^x(dP)]  (scc_routine.rs:176-183; helpers.rs:111-155)
 template <class T>
 __device__ void sc_fock(int n, int N, bool lc, const ScWork<T> &w, const double *p0, ScShared &sm) {
-    const int tid = threadIdx.x;
     const long long nn = (long long)n * n;
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         const T es = (T)(0.5 * (sm.esp[sm.ao_atom[mu]] + sm.esp[sm.ao_atom[nu]]));
         w.F[t] = fma(es, w.S[t], w.H0[t]);
     }
     if (!lc) {
-        __syncthreads();
+        sc_bar(sm);
         return;
     }
     T *dP = w.W, *hx = w.W + nn, *tmp = w.W + 2 * nn;
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         dP[t] = w.P[t] - (mu == nu ? (T)p0[mu] : T(0));
     }
-    __syncthreads();
+    sc_bar(sm);
 #define GLR(mu, nu) w.glr[(long long)sm.ao_atom[mu] * N + sm.ao_atom[nu]]
     gemm<T>(n, n, n, T(1), w.S, n, false, dP, n, false, T(0), w.T1, n, sm);   // S dP
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         tmp[t] = GLR(mu, nu) * w.T1[t];
     }
-    __syncthreads();
+    sc_bar(sm);
     gemm<T>(n, n, n, T(1), tmp, n, false, w.S, n, false, T(0), w.T2, n, sm);   // (g o S dP) S
     gemm_sym<T>(n, n, T(1), w.T1, n, false, w.S, n, false, T(0), w.T3, n, sm);   // S dP S
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         const T g = GLR(mu, nu);
         hx[t] = w.T2[t] + w.T2[(long long)nu * n + mu] + g * w.T3[t];
         tmp[t] = dP[t] * g;
     }
-    __syncthreads();
+    sc_bar(sm);
     gemm<T>(n, n, n, T(1), w.S, n, false, tmp, n, false, T(0), w.T1, n, sm);   // S (dP o g)
     gemm_sym<T>(n, n, T(1), w.T1, n, false, w.S, n, false, T(1), hx, n, sm);    // + S (dP o g) S
-    for (long long t = tid; t < nn; t += SC_T) {
+    SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         w.F[t] += T(-0.0625) * (hx[t] + hx[(long long)nu * n + mu]);
     }
 #undef GLR
-    __syncthreads();
+    sc_bar(sm);
 }
 
 // solve the DIIS equations (m + 1 unknowns, the last the multiplier) on thread 0; sm.coef
@@ -823,7 +1013,7 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
         T *Fc = w.Fh + cur * nn, *Ec = w.Eh + cur * nn;
         double emax = 0.0;
         bool fin = true;
-        for (long long t = tid; t < nn; t += SC_T) {
+        SC_FOR(t, nn) {
             const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
             const T ev = w.T1[t] - w.T1[(long long)nu * n + mu];
             Ec[t] = ev;
@@ -847,7 +1037,7 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
         {
             double v[SC_DIIS];
             for (int i = 0; i < m; ++i) v[i] = 0.0;
-            for (long long t = tid; t < nn; t += SC_T) {
+            SC_FOR(t, nn) {
                 const double ec = (double)Ec[t];
                 for (int i = 0; i < m; ++i) v[i] = fma((double)w.Eh[i * nn + t], ec, v[i]);
             }
@@ -865,7 +1055,7 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
             sm.coef[cur] = 1.0;
         }
         __syncthreads();
-        for (long long t = tid; t < nn; t += SC_T) {
+        SC_FOR(t, nn) {
             T v = T(0);
             if (m > 1) {
                 for (int i = 0; i < m; ++i) v = fma((T)sm.coef[i], w.Fh[i * nn + t], v);
@@ -878,7 +1068,7 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
             }
             w.EA[t] = v;
         }
-        __syncthreads();
+        sc_bar(sm);
         if (!sc_eigh<T>(n, o, w.EA, w.Z, w.W, piv, sm)) {
             st.finite = false;
             return;
@@ -893,12 +1083,22 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
 __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
     __shared__ ScShared sm;
     const int tid = threadIdx.x;
-    const ScSlot sl = sc_slot(a, blockIdx.x);
+    const ScSlot sl = sc_slot(a, blockIdx.x / a.csize);
+    if (tid == 0) {
+        sm.rank = blockIdx.x % a.csize;
+        sm.csize = a.csize;
+        sm.par = 0;
+    }
+    __syncthreads();
+    sc_bar(sm);   // every CTA of the cluster runs before the first access to its shared memory
     for (int guard = 0; guard < a.n_sys; ++guard) {
-        if (tid == 0) sm.sys_id = atomicAdd(a.next, 1);
-        __syncthreads();
+        if (tid == 0 && sm.rank == 0) {
+            const int nx = atomicAdd(a.next, 1);
+            for (int c = 0; c < a.csize; ++c) *(a.csize > 1 ? sc_at(&sm.sys_id, c) : &sm.sys_id) = nx;
+        }
+        sc_bar(sm);
         const int q = sm.sys_id;
-        __syncthreads();
+        sc_bar(sm);
         if (q >= a.n_sys) break;
         const int id = a.order[q];
         const tincr_scc_system sy = a.sys[id];
@@ -906,7 +1106,7 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
         const long long nn = (long long)n * n, NN = (long long)N * N;
         const double erep = sc_setup(a, sy, sl, sm);
         const double *p0 = sl.p0;
-        for (int mu = tid; mu < n; mu += SC_T) {
+        SC_FOR(mu, n) {
             const int A = sm.ao_atom[mu];
             sl.p0[mu] = a.kind_occ[4 * sm.kind[A] + (mu - sm.ao_off[A])];
         }
@@ -914,29 +1114,29 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
         ScWork<double> w = sc_work<double>(sl, nn);
         w.S = sl.S; w.H0 = sl.H0; w.X = sl.X; w.Sh = sl.Sh; w.gam = sl.gam; w.glr = sl.glr;
         // X = S^-1/2 and S^1/2 from the eigenpairs of S (scc_routine.rs:172-174)
-        for (long long t = tid; t < nn; t += SC_T) w.EA[t] = w.S[t];
-        __syncthreads();
+        SC_FOR(t, nn) w.EA[t] = w.S[t];
+        sc_bar(sm);
         bool ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, sm);
         if (ok) {
             double bad = 0.0;
             for (int r = tid; r < n; r += SC_T) bad = fmax(bad, sm.w[r] > 0.0 ? 0.0 : 1.0);
-            ok = sc_max(bad, sm) == 0.0;
+            ok = sc_max_cta(bad, sm) == 0.0;
         }
         const double *ps = a.p_start ? a.p_start + sy.mat_off : nullptr;
         auto start_density = [&]() {
-            for (long long t = tid; t < nn; t += SC_T) {
+            SC_FOR(t, nn) {
                 const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
                 w.P[t] = ps ? ps[t] : (mu == nu ? p0[mu] : 0.0);
             }
-            __syncthreads();
+            sc_bar(sm);
         };
         if (ok) {
-            for (long long t = tid; t < nn; t += SC_T) {
+            SC_FOR(t, nn) {
                 const int r = (int)(t % n);
                 w.T1[t] = w.Z[t] / sqrt(sm.w[r]);
                 w.T2[t] = w.Z[t] * sqrt(sm.w[r]);
             }
-            __syncthreads();
+            sc_bar(sm);
             gemm_sym<double>(n, n, 1.0, w.T1, n, false, w.Z, n, true, 0.0, w.X, n, sm);
             gemm_sym<double>(n, n, 1.0, w.T2, n, false, w.Z, n, true, 0.0, w.Sh, n, sm);
             start_density();
@@ -949,18 +1149,18 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
             float *cp = reinterpret_cast<float *>(sl.work) + (13 + 2 * SC_DIIS) * nn;
             wf.S = cp; wf.H0 = cp + nn; wf.X = cp + 2 * nn; wf.Sh = cp + 3 * nn; wf.gam = cp + 4 * nn;
             wf.glr = wf.gam + NN;
-            for (long long t = tid; t < nn; t += SC_T) {
+            SC_FOR(t, nn) {
                 wf.S[t] = (float)w.S[t];
                 wf.H0[t] = (float)w.H0[t];
                 wf.X[t] = (float)w.X[t];
                 wf.Sh[t] = (float)w.Sh[t];
                 wf.P[t] = (float)w.P[t];
             }
-            for (long long t = tid; t < NN; t += SC_T) {
+            SC_FOR(t, NN) {
                 wf.gam[t] = (float)w.gam[t];
                 wf.glr[t] = (float)w.glr[t];
             }
-            __syncthreads();
+            sc_bar(sm);
             const int lim = remaining < SC_FP32_MAX ? remaining : SC_FP32_MAX;
             ScState sf{0, false, 0.0, true};
             sc_iterate<float>(a, sy, wf, sl.piv, p0, lim, fmax(a.tol, SC_FP32_SWITCH), sf, hist, sm);
@@ -968,12 +1168,12 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
                 // continue in FP64 from the density of the FP32 phase's last diagonalisation, with
                 // its DIIS history: E' first (FP64 slots beyond every FP32 array), then F' (FP64
                 // slots over the FP32 E' and input copies, which are done with)
-                for (long long t = tid; t < nn; t += SC_T) w.P[t] = (double)wf.P[t];
+                SC_FOR(t, nn) w.P[t] = (double)wf.P[t];
                 const int m = hist + 1 < SC_DIIS ? hist + 1 : SC_DIIS;
-                for (long long t = tid; t < m * nn; t += SC_T) w.Eh[t] = (double)wf.Eh[t];
-                __syncthreads();
-                for (long long t = tid; t < m * nn; t += SC_T) w.Fh[t] = (double)wf.Fh[t];
-                __syncthreads();
+                SC_FOR(t, m * nn) w.Eh[t] = (double)wf.Eh[t];
+                sc_bar(sm);
+                SC_FOR(t, m * nn) w.Fh[t] = (double)wf.Fh[t];
+                sc_bar(sm);
             } else {
                 start_density();
                 hist = 0;
@@ -997,8 +1197,8 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
         double energy = 0.0;
         if (ok) {
             // orbitals of the last Fock matrix (scc_routine.rs:187-192)
-            for (long long t = tid; t < nn; t += SC_T) w.EA[t] = w.Fp[t];
-            __syncthreads();
+            SC_FOR(t, nn) w.EA[t] = w.Fp[t];
+            sc_bar(sm);
             ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, sm);
         }
         if (ok) {
@@ -1008,20 +1208,20 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
             sc_charges<double>(n, N, w.P, w.S, w.gam, p0, sm);
             // E = sum P o H0 + 1/2 dq gamma dq [- 1/8 (sum (S dP S) o dP o g_lr + sum (S dP) o (dP S) o g_lr)]
             double e1 = 0.0;
-            for (long long t = tid; t < nn; t += SC_T) e1 = fma(w.P[t], w.H0[t], e1);
+            SC_FOR(t, nn) e1 = fma(w.P[t], w.H0[t], e1);
             double e2 = 0.0;
-            for (int A = tid; A < N; A += SC_T) e2 += 0.5 * sm.dq[A] * sm.esp[A];
+            SC_FOR(A, N) e2 += 0.5 * sm.dq[A] * sm.esp[A];
             double e3 = 0.0;
             if (a.lc) {
                 double *dP = w.W;
-                for (long long t = tid; t < nn; t += SC_T) {
+                SC_FOR(t, nn) {
                     const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
                     dP[t] = w.P[t] - (mu == nu ? p0[mu] : 0.0);
                 }
-                __syncthreads();
+                sc_bar(sm);
                 gemm<double>(n, n, n, 1.0, w.S, n, false, dP, n, false, 0.0, w.T1, n, sm);
                 gemm_sym<double>(n, n, 1.0, w.T1, n, false, w.S, n, false, 0.0, w.T2, n, sm);
-                for (long long t = tid; t < nn; t += SC_T) {
+                SC_FOR(t, nn) {
                     const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
                     const double g = w.glr[(long long)sm.ao_atom[mu] * N + sm.ao_atom[nu]];
                     e3 += g * (w.T2[t] * dP[t] + w.T1[t] * w.T1[(long long)nu * n + mu]);
@@ -1029,23 +1229,23 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
                 e3 *= -0.125;
             }
             energy = sc_sum(e1 + e2 + e3, sm) + erep;
-            for (int r = tid; r < n; r += SC_T) a.orbe[sy.orb_off + r] = sm.w[r];
-            for (int A = tid; A < N; A += SC_T) a.dq[sy.atom_off + A] = sm.dq[A];
-            for (long long t = tid; t < nn; t += SC_T) {
+            SC_FOR(r, n) a.orbe[sy.orb_off + r] = sm.w[r];
+            SC_FOR(A, N) a.dq[sy.atom_off + A] = sm.dq[A];
+            SC_FOR(t, nn) {
                 if (a.p) a.p[sy.mat_off + t] = w.P[t];
                 if (a.s_out) a.s_out[sy.mat_off + t] = w.S[t];
                 if (a.h0_out) a.h0_out[sy.mat_off + t] = w.H0[t];
                 if (a.hcx) a.hcx[sy.mat_off + t] = w.F[t];
             }
         }
-        if (tid == 0) {
+        if (tid == 0 && sm.rank == 0) {
             a.iterations[id] = st.it;
             a.converged[id] = (ok && st.converged) ? 1 : 0;
             a.residual[id] = ok ? st.errn : NAN;
             a.energy[id] = ok ? energy : NAN;
             a.status[id] = ok ? TINCR_OK : TINCR_NONFINITE;
         }
-        __syncthreads();
+        sc_bar(sm);
     }
 }
 
@@ -1137,7 +1337,10 @@ int Ctx::scc_batch(int n_sys, const tincr_scc_system *sys, const int *kinds, con
     const long long nn_max = (long long)nmax * nmax, at2_max = (long long)Nmax * Nmax, npad = (nmax + 31) / 32 * 32;
     const long long slot_bytes =
         (sc_slot_doubles(nn_max, at2_max, npad) * (long long)sizeof(double) + nn_max + 255) / 256 * 256;
-    const int n_slots = std::min(n_sys, SC_SLOTS_PER_SM * n_sm);
+    // CTAs per system
+    int csize = 1;
+    while (csize < SC_CMAX && 2LL * csize * n_sys <= SC_FILL * n_sm) csize *= 2;
+    const int n_slots = std::min(n_sys, SC_SLOTS_PER_SM * n_sm / csize);
     scc_ws.reserve((size_t)(slot_bytes * n_slots));
     ScArgs a{};
     a.n_sys = n_sys;
@@ -1193,7 +1396,19 @@ int Ctx::scc_batch(int n_sys, const tincr_scc_system *sys, const int *kinds, con
     a.npad = npad;
     TINCR_CUDA(cudaEventRecord(ev0, stream));
     g_launches = 0;
-    scc_kernel<<<n_slots, SC_T, 0, stream>>>(a);
+    a.csize = csize;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(n_slots * csize));
+    cfg.blockDim = dim3(SC_T);
+    cfg.stream = stream;
+    cudaLaunchAttribute cl[1];
+    cl[0].id = cudaLaunchAttributeClusterDimension;
+    cl[0].val.clusterDim.x = (unsigned)csize;
+    cl[0].val.clusterDim.y = cl[0].val.clusterDim.z = 1;
+    cfg.attrs = cl;
+    cfg.numAttrs = 1;
+    if (csize > 8) TINCR_CUDA(cudaFuncSetAttribute(scc_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    TINCR_CUDA(cudaLaunchKernelEx(&cfg, scc_kernel, a));
     count_launch(stream, "scc_kernel");
     check_launch("scc_kernel");
     TINCR_CUDA(cudaEventRecord(ev1, stream));
