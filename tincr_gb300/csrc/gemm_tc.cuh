@@ -3,17 +3,19 @@
 // C[M x N] = A[M x K] B[N x K]^T with A and B in three split-BF16 planes each (planes.cuh),
 // accumulated as the six plane products A0B0 + A0B1 + A1B0 + A0B2 + A2B0 + A1B1.
 //
-// Persistent: at most one CTA per SM, each walking the 128 x 128 output tiles t = blockIdx.x,
+// Persistent: at most one CTA per SM, each walking the 128 x TN output tiles t = blockIdx.x,
 // + gridDim.x, ... (all roles in the same order), so the loads and MMAs of a tile's first K blocks
-// overlap the previous tile's epilogue.  CTA = 320 threads, K consumed in 64-element (128-byte) blocks:
-//   * warp 8 / lane 0: TMA producer, six boxes (A0, A1, A2, B0, B1, B2; 128 rows x 64 bf16, 128-byte
-//     swizzle) per stage into a 2-stage ring, completion on the stage's "full" mbarrier;
-//   * warp 9 / lane 0: MMA issuer, 4 K=16 steps x 6 products per block (tcgen05.mma.cta_group::1
-//     .kind::f16, M = N = 128) into one of two TMEM accumulator pairs (ping-pong): the hi x hi product
+// overlap the previous tile's epilogue.  TN is 128, 64 or 32 (tc_tile_for).  K is consumed in 64-element
+// (128-byte) blocks; for TN = 128 (TN = 32: 8 fold warps):
+//   * warp 16 / lane 0: TMA producer, six boxes (A0, A1, A2 of 128 rows, B0, B1, B2 of TN rows, 64 bf16
+//     each, 128-byte swizzle) per stage into a ring of 2 (TN < 128: 3) stages, completion on the
+//     stage's "full" mbarrier;
+//   * warp 17 / lane 0: MMA issuer, 4 K=16 steps x 6 products per block (tcgen05.mma.cta_group::1
+//     .kind::f16, M = 128, N = TN) into one of two TMEM accumulator pairs (ping-pong): the hi x hi product
 //     in one accumulator, the five smaller products in the other; tcgen05.commit to the stage's
 //     "empty" and the pair's "full" mbarrier;
-//   * warps 0-7: fold each K block's pair into FP32 running sums held in registers (warp w owns
-//     TMEM lanes 32 (w % 4) .. + 31 = tile rows, one row per thread, and columns 64 (w / 4) .. + 63),
+//   * warps 0-15: fold each K block's pair into FP32 running sums held in registers (warp w owns
+//     TMEM lanes 32 (w % 4) .. + 31 = tile rows, one row per thread, and columns 32 (w / 4) .. + 31),
 //     then the epilogue functor.
 // The dominant accumulator takes only 4 MMAs per block before the CUDA cores add it with
 // round-to-nearest, and the small products accumulate apart from it, which keeps long K (up to
@@ -30,18 +32,27 @@
 
 namespace tincr {
 
-constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 2, TC_T = 320;
-constexpr int TC_FOLD_WARPS = 8;                         // warps 0-7 fold and run the epilogue
-constexpr int TC_TILE = TC_M * TC_K * 2;                  // 16 KB (128 rows x 128 bytes)
-constexpr int TC_STAGE = 2 * N_PLANES * TC_TILE;          // A0, A1, A2, B0, B1, B2
-constexpr int TC_SMEM = TC_STAGES * TC_STAGE + 1024 + 256;
-constexpr int TC_COLS = 4 * TC_N;                         // two ping-pong pairs {hi x hi, other products}
+constexpr int TC_M = 128, TC_K = 64;
+constexpr int TC_TILE = TC_M * TC_K * 2;                  // 16 KB (128 rows x 128 bytes): one A plane
 constexpr unsigned long long TC_WAIT_NS = 2000000000ull;  // a wait gives up after 2 s
 
-// instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
-// both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28
-constexpr uint32_t TC_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_N >> 3) << 17) |
-                              ((uint32_t)(TC_M >> 4) << 24);
+// A tile of 128 x TN outputs: fold and epilogue warps, stages of the TMA ring, shared memory, TMEM
+template <int TN>
+struct TcTile {
+    static constexpr int N = TN;
+    static constexpr int FOLD_WARPS = TN == 32 ? 8 : 16;          // four lane quarters x FOLD_WARPS / 4 column ranges
+    static constexpr int HN = TN / (FOLD_WARPS / 4);              // columns per fold warp: 16 or 32
+    static constexpr int T = 32 * (FOLD_WARPS + 2);
+    static constexpr int STAGES = TN == 128 ? 2 : 3;
+    static constexpr int BTILE = TN * TC_K * 2;                   // one B plane
+    static constexpr int STAGE = N_PLANES * (TC_TILE + BTILE);    // A0, A1, A2, B0, B1, B2
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+    static constexpr int COLS = 4 * TN;                           // two ping-pong pairs {hi x hi, other products}
+    // instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
+    // both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
+                                      ((uint32_t)(TC_M >> 4) << 24);
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -93,11 +104,11 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-        "l"(adesc), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
@@ -128,47 +139,49 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr));
 }
 
+constexpr double TC_OVERHEAD = 32.0;   // of a tile, in columns (tc_tile_for)
+
 // tensor maps of the three A planes, then the three B planes
 struct TcMaps {
     CUtensorMap m[2 * N_PLANES];
 };
 
-template <class Epi>
-__global__ void __launch_bounds__(TC_T, 1)
+template <class W, class Epi>
+__global__ void __launch_bounds__(W::T, 1)
 gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpad, int a_batched, int b_batched,
                       int batch, Epi epi, int *err, unsigned long long first_wait_ns) {
     extern __shared__ unsigned char tc_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + TC_STAGES * TC_STAGE);
-    uint64_t *empty = full + TC_STAGES;
-    uint64_t *accf = empty + TC_STAGES;      // accumulator a holds a finished K block
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + W::STAGES * W::STAGE);
+    uint64_t *empty = full + W::STAGES;
+    uint64_t *accf = empty + W::STAGES;      // accumulator a holds a finished K block
     uint64_t *acce = accf + 2;               // accumulator a has been folded
     uint64_t *done = acce + 2;               // every MMA issued has completed
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nk = Kpad / TC_K;
-    const int tiles_n = (N + TC_N - 1) / TC_N, tiles_m = (M + TC_M - 1) / TC_M;
+    const int tiles_n = (N + W::N - 1) / W::N, tiles_m = (M + TC_M - 1) / TC_M;
     const int n_tiles = tiles_n * tiles_m * batch;
     // tile t = (b tiles_m + mt) tiles_n + nt; this CTA takes t = blockIdx.x, + gridDim.x, ...  Every
     // role walks the same tiles and K blocks; g counts this CTA's K blocks over all its tiles and
-    // gives the stage (g % TC_STAGES), the accumulator pair (g & 1) and the barrier phases.
+    // gives the stage (g % W::STAGES), the accumulator pair (g & 1) and the barrier phases.
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) {
+        for (int s = 0; s < W::STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&accf[a], 1);
-            mbar_init(&acce[a], TC_FOLD_WARPS);   // one arrival per folding warp
+            mbar_init(&acce[a], W::FOLD_WARPS);   // one arrival per folding warp
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
-                     "r"(TC_COLS));
+                     "r"(W::COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -176,45 +189,45 @@ gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpa
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == TC_FOLD_WARPS) {
+    if (warp == W::FOLD_WARPS) {
         if (lane == 0) {
             long long g = 0, issued = 0;
             bool ok = true;
             for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
                 const int nt = t % tiles_n, mt = (t / tiles_n) % tiles_m, b = t / (tiles_n * tiles_m);
-                const int m0 = mt * TC_M, n0 = nt * TC_N;
+                const int m0 = mt * TC_M, n0 = nt * W::N;
                 for (int kb = 0; kb < nk; ++kb, ++g) {
-                    const int s = (int)(g % TC_STAGES);
-                    if (g >= TC_STAGES && !mbar_wait(&empty[s], (unsigned)((g / TC_STAGES) & 1) ^ 1u)) {
+                    const int s = (int)(g % W::STAGES);
+                    if (g >= W::STAGES && !mbar_wait(&empty[s], (unsigned)((g / W::STAGES) & 1) ^ 1u)) {
                         atomicExch(err, 1);
                         ok = false;
                         break;
                     }
-                    unsigned char *st = smem + s * TC_STAGE;
-                    mbar_expect_tx(&full[s], TC_STAGE);
+                    unsigned char *st = smem + s * W::STAGE;
+                    mbar_expect_tx(&full[s], W::STAGE);
 #pragma unroll
                     for (int q = 0; q < N_PLANES; ++q) {
                         tma_load_3d(st + q * TC_TILE, &maps.m[q], kb * TC_K, m0, a_batched ? b : 0, &full[s]);
-                        tma_load_3d(st + (N_PLANES + q) * TC_TILE, &maps.m[N_PLANES + q], kb * TC_K, n0,
+                        tma_load_3d(st + N_PLANES * TC_TILE + q * W::BTILE, &maps.m[N_PLANES + q], kb * TC_K, n0,
                                     b_batched ? b : 0, &full[s]);
                     }
                     issued = g + 1;
                 }
             }
             if (!ok)   // loads still in flight land before the CTA exits
-                for (long long h = (issued > TC_STAGES ? issued - TC_STAGES : 0); h < issued; ++h)
-                    mbar_wait(&full[h % TC_STAGES], (unsigned)((h / TC_STAGES) & 1));
+                for (long long h = (issued > W::STAGES ? issued - W::STAGES : 0); h < issued; ++h)
+                    mbar_wait(&full[h % W::STAGES], (unsigned)((h / W::STAGES) & 1));
         }
-    } else if (warp == TC_FOLD_WARPS + 1) {
+    } else if (warp == W::FOLD_WARPS + 1) {
         if (lane == 0) {
             long long g = 0;
             bool ok = true;
             for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
                 for (int kb = 0; kb < nk; ++kb, ++g) {
-                    const int s = (int)(g % TC_STAGES), a = (int)(g & 1);
+                    const int s = (int)(g % W::STAGES), a = (int)(g & 1);
                     // first_wait_ns limits the first of these waits (TC_WAIT_NS unless a test shortens it
                     // to exercise the recovery: the producer drains its loads, the fold warps give up)
-                    if (!mbar_wait(&full[s], (unsigned)((g / TC_STAGES) & 1), g == 0 ? first_wait_ns : TC_WAIT_NS)) {
+                    if (!mbar_wait(&full[s], (unsigned)((g / W::STAGES) & 1), g == 0 ? first_wait_ns : TC_WAIT_NS)) {
                         atomicExch(err, 2);
                         ok = false;
                         break;
@@ -225,21 +238,21 @@ gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpa
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t base = smem_u32(smem + s * TC_STAGE);
-                    const uint32_t dm = tmem + (uint32_t)(a * 2 * TC_N), dx = dm + (uint32_t)TC_N;
+                    const uint32_t base = smem_u32(smem + s * W::STAGE);
+                    const uint32_t dm = tmem + (uint32_t)(a * 2 * W::N), dx = dm + (uint32_t)W::N;
 #pragma unroll
                     for (int kk = 0; kk < TC_K / 16; ++kk) {
                         const uint32_t off = kk * 32;   // 16 bf16 = 32 bytes along K
                         const uint64_t a0 = tc_desc(base + 0 * TC_TILE + off), a1 = tc_desc(base + 1 * TC_TILE + off),
                                        a2 = tc_desc(base + 2 * TC_TILE + off);
-                        const uint64_t b0 = tc_desc(base + 3 * TC_TILE + off), b1 = tc_desc(base + 4 * TC_TILE + off),
-                                       b2 = tc_desc(base + 5 * TC_TILE + off);
-                        tc_mma(dm, a0, b0, kk > 0 ? 1u : 0u);
-                        tc_mma(dx, a0, b1, kk > 0 ? 1u : 0u);
-                        tc_mma(dx, a1, b0, 1u);
-                        tc_mma(dx, a0, b2, 1u);
-                        tc_mma(dx, a2, b0, 1u);
-                        tc_mma(dx, a1, b1, 1u);
+                        const uint32_t bb = base + N_PLANES * TC_TILE + off;
+                        const uint64_t b0 = tc_desc(bb), b1 = tc_desc(bb + W::BTILE), b2 = tc_desc(bb + 2 * W::BTILE);
+                        tc_mma(dm, a0, b0, W::IDESC, kk > 0 ? 1u : 0u);
+                        tc_mma(dx, a0, b1, W::IDESC, kk > 0 ? 1u : 0u);
+                        tc_mma(dx, a1, b0, W::IDESC, 1u);
+                        tc_mma(dx, a0, b2, W::IDESC, 1u);
+                        tc_mma(dx, a2, b0, W::IDESC, 1u);
+                        tc_mma(dx, a1, b1, W::IDESC, 1u);
                     }
                     tc_commit(&empty[s]);
                     tc_commit(&accf[a]);
@@ -249,16 +262,16 @@ gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpa
             mbar_wait(done, 0);   // no MMA is in flight once the issuer leaves (also after a failure)
         }
     } else {
-        // folding warps 0-7: row m0 + 32 (warp % 4) + lane (TMEM lane quarter of the warp), columns
-        // n0 + 64 (warp / 4) .. + 63: two warps per lane quarter halve the fold and epilogue per thread.
+        // folding warps: row m0 + 32 (warp % 4) + lane (TMEM lane quarter of the warp), columns
+        // n0 + HN (warp / 4) .. + HN - 1: several warps per lane quarter share the fold and the epilogue.
         // A tile's epilogue runs while the MMAs of the next tile's first K blocks proceed.
-        constexpr int HN = TC_N / 2;
+        constexpr int HN = W::HN;
         const int quarter = warp & 3, half = warp >> 2;
         long long g = 0;
         bool ok = true;
         for (int t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
             const int nt = t % tiles_n, mt = (t / tiles_n) % tiles_m, b = t / (tiles_n * tiles_m);
-            const int m0 = mt * TC_M, n0 = nt * TC_N;
+            const int m0 = mt * TC_M, n0 = nt * W::N;
             float sum[HN];
 #pragma unroll
             for (int j = 0; j < HN; ++j) sum[j] = 0.f;
@@ -271,12 +284,12 @@ gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpa
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t t0 =
-                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * 2 * TC_N) + (uint32_t)(half * HN);
+                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * 2 * W::N) + (uint32_t)(half * HN);
 #pragma unroll
                 for (int c0 = 0; c0 < HN; c0 += 16) {
                     uint32_t rm[16], rx[16];
                     tmem_ld16(t0 + (uint32_t)c0, rm);
-                    tmem_ld16(t0 + (uint32_t)(TC_N + c0), rx);
+                    tmem_ld16(t0 + (uint32_t)(W::N + c0), rx);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(rm[j]) + __uint_as_float(rx[j]);
@@ -301,7 +314,7 @@ gemm_planes_tc_kernel(const __grid_constant__ TcMaps maps, int M, int N, int Kpa
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC_COLS));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(W::COLS));
     }
 }
 
@@ -321,14 +334,15 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// 3-D map over bf16 planes [batch][rows][ld] with logical extent [batch][rows][Kpad], box 64 x 128
-inline CUtensorMap plane_map(const bf16 *base, int rows, long long Kpad, long long ld, long long sb, int batch) {
+// 3-D map over bf16 planes [batch][rows][ld] with logical extent [batch][rows][Kpad], box 64 x box_rows
+inline CUtensorMap plane_map(const bf16 *base, int rows, long long Kpad, long long ld, long long sb, int batch,
+                             int box_rows) {
     if (((uintptr_t)base & 15) || (ld * 2) % 16 || (sb * 2) % 16 || Kpad % TC_K)
         fail(TINCR_BAD_ARG, "plane_map: alignment");
     CUtensorMap m;
     cuuint64_t dims[3] = {(cuuint64_t)Kpad, (cuuint64_t)rows, (cuuint64_t)(sb ? batch : 1)};
     cuuint64_t strides[2] = {(cuuint64_t)(ld * 2), (cuuint64_t)((sb ? sb : ld * rows) * 2)};
-    cuuint32_t box[3] = {TC_K, TC_M, 1};
+    cuuint32_t box[3] = {TC_K, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = tensor_map_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16 *>(base), dims, strides,
                                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -337,29 +351,63 @@ inline CUtensorMap plane_map(const bf16 *base, int rows, long long Kpad, long lo
     return m;
 }
 
+template <class W, class Epi>
+void gemm_planes_tc_launch(cudaStream_t st, int M, int N, int Kpad, const PlaneOperand &A, const PlaneOperand &B,
+                           int batch, const Epi &epi, int *d_err, int n_sm, unsigned long long first_wait_ns) {
+    TcMaps maps;
+    for (int q = 0; q < N_PLANES; ++q) {
+        maps.m[q] = plane_map(A.p + q * A.ps, M, Kpad, A.ld, A.sb, batch, TC_M);
+        maps.m[N_PLANES + q] = plane_map(B.p + q * B.ps, N, Kpad, B.ld, B.sb, batch, W::N);
+    }
+    static bool attr = false;
+    if (!attr) {
+        TINCR_CUDA(cudaFuncSetAttribute(gemm_planes_tc_kernel<W, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, W::SMEM));
+        attr = true;
+    }
+    // persistent: at most one CTA per SM (the shared memory allows one), each walking its tiles
+    const long long n_tiles = (long long)ceil_div(N, W::N) * ceil_div(M, TC_M) * batch;
+    if (n_tiles > (1LL << 31) - 1) fail(TINCR_BAD_ARG, "gemm_planes_tc: too many tiles");
+    const int grid = (int)std::min<long long>(n_tiles, std::max(1, n_sm));
+    gemm_planes_tc_kernel<W, Epi><<<grid, W::T, W::SMEM, st>>>(maps, M, N, Kpad, A.sb ? 1 : 0, B.sb ? 1 : 0, batch, epi,
+                                                               d_err, first_wait_ns);
+    count_launch(st, "gemm_planes_tc");
+    check_launch("gemm_planes_tc");
+}
+
+// Columns of the output tile: the width with the least (waves of tiles over the SMs) x (TN +
+// TC_OVERHEAD), a tile's cost being its columns (MMAs, fold, epilogue) and a fixed part (the A planes).
+// The sums of an output do not depend on the width, so results are bit for bit the same.  128 columns
+// alone left a small product on a few SMs, whose epilogues (FP64 stores and conversions) then took
+// longest: S0 + S1 gradient, 128 only / this rule, ms on the device: (H2O)48 7.6 / 5.9, decacene 7.3 /
+// 5.3, pentacene 5.9 / 4.7; 5 products of (H2O)64 0.177 / 0.127; 20 products of (H2O)128 0.83 / 0.83 (32
+// columns: 1.17).  Overheads of 32, 64 and 128 measured alike but for (H2O)64 (0.127, 0.134, 0.128).
+inline int tc_tile_for(int M, int N, int batch, int n_sm) {
+    int best = 128;
+    double cost = 0.0;
+    for (int tn = 128; tn >= 32; tn /= 2) {
+        const long long tiles = (long long)ceil_div(M, TC_M) * ceil_div(N, tn) * batch;
+        const double c = (double)((tiles + n_sm - 1) / n_sm) * (TC_OVERHEAD + tn);
+        if (tn == 128 || c < cost) {
+            best = tn;
+            cost = c;
+        }
+    }
+    return best;
+}
+
 template <class Epi>
 void gemm_planes_tc(cudaStream_t st, int M, int N, int Kpad, PlaneOperand A, PlaneOperand B, int batch, Epi epi,
                     int *d_err, int n_sm, unsigned long long first_wait_ns = TC_WAIT_NS) {
     if (M <= 0 || N <= 0 || batch <= 0) return;
     if (Kpad <= 0 || Kpad % TC_K) fail(TINCR_BAD_ARG, "gemm_planes_tc: K not padded to 64");
-    TcMaps maps;
-    for (int q = 0; q < N_PLANES; ++q) {
-        maps.m[q] = plane_map(A.p + q * A.ps, M, Kpad, A.ld, A.sb, batch);
-        maps.m[N_PLANES + q] = plane_map(B.p + q * B.ps, N, Kpad, B.ld, B.sb, batch);
+    auto go = [&](auto w) {
+        gemm_planes_tc_launch<decltype(w)>(st, M, N, Kpad, A, B, batch, epi, d_err, n_sm, first_wait_ns);
+    };
+    switch (tc_tile_for(M, N, batch, std::max(1, n_sm))) {
+        case 128: go(TcTile<128>{}); break;
+        case 64: go(TcTile<64>{}); break;
+        default: go(TcTile<32>{}); break;
     }
-    static bool attr = false;
-    if (!attr) {
-        TINCR_CUDA(cudaFuncSetAttribute(gemm_planes_tc_kernel<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
-        attr = true;
-    }
-    // persistent: at most one CTA per SM (the shared memory allows one), each walking its tiles
-    const long long n_tiles = (long long)ceil_div(N, TC_N) * ceil_div(M, TC_M) * batch;
-    if (n_tiles > (1LL << 31) - 1) fail(TINCR_BAD_ARG, "gemm_planes_tc: too many tiles");
-    const int grid = (int)std::min<long long>(n_tiles, std::max(1, n_sm));
-    gemm_planes_tc_kernel<Epi><<<grid, TC_T, TC_SMEM, st>>>(maps, M, N, Kpad, A.sb ? 1 : 0, B.sb ? 1 : 0, batch, epi,
-                                                            d_err, first_wait_ns);
-    count_launch(st, "gemm_planes_tc");
-    check_launch("gemm_planes_tc");
 }
 
 }  // namespace tincr
