@@ -118,6 +118,8 @@ struct Ctx {
     void tc_err_watch();                  // queue the copy of d_tc_err to h_tc_err (checked at the next sync)
 
     // product workspace
+    DevBuf<double> px;                     // X as given, transposed, A.X of the last tincr_tda_products call
+    DevBuf<int> px_bad;
     DevBuf<double> wsH, wsF, wsG, wsd3, wsd2, wsz;
     // Davidson state
     DevBuf<double> dV, dAV, dR, dRk, dT;
@@ -166,7 +168,7 @@ struct Ctx {
     DevBuf<int> gs_state;
     int coop_grid = 0;                    // CTAs of the cooperative Gram-Schmidt launch
     void row_norms(int rows, long long len, const double *A, long long lda, double *out);
-    void launch_transpose(int rows, int cols, const double *in, double *out);
+    void launch_transpose(int rows, int cols, const double *in, double *out, int *bad = nullptr);
     void set_atoms(int n_atoms, const int *orbs_per_atom, int n_orb);
     void upload_mo(int n, const double *C, const double *S);
     int product_chunk() const;
