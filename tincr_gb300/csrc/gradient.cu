@@ -107,26 +107,25 @@ __global__ void w_assemble_kernel(int o, int v, const double *wij, const double 
     }
 }
 
-// sv[b] = sum_a S[a][b] (V[a][b] + V[b][a]),  r[a] = sum_b S[a][b] (Y[a][b] + Y[b][a])  (S symmetric)
+// sv[b] = sum_a S[a][b] (V[a][b] + V[b][a]),  r[a] = sum_b S[a][b] (Y[a][b] + Y[b][a])  (S symmetric):
+// one warp per entry (one thread per entry read its row of S with a stride of n: 134 us at n = 288)
 __global__ void fv_vectors_kernel(int n, const double *S, const double *V, const double *Y, double *sv, double *r) {
-    GRID_STRIDE(t, 2LL * n) {
-        int k = int(t % n);
-        const double *s = S + (long long)k * n;
-        double acc = 0.0;
-        if (t < n) {
-            for (int a = 0; a < n; ++a) acc += s[a] * (V[(long long)a * n + k] + V[(long long)k * n + a]);
-            sv[k] = acc;
-        } else {
-            for (int b = 0; b < n; ++b) acc += s[b] * (Y[(long long)k * n + b] + Y[(long long)b * n + k]);
-            r[k] = acc;
-        }
-    }
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (e >= 2 * n) return;
+    const int k = e < n ? e : e - n;
+    const double *s = S + (long long)k * n, *M = e < n ? V : Y;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int a = lane; a < n; a += 32) acc += s[a] * (M[(long long)a * n + k] + M[(long long)k * n + a]);
+    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane == 0) (e < n ? sv : r)[k] = acc;
 }
 
-// per-atom sums of an AO vector and their gamma products:  out_ao[mu] = sum_B g[A(mu)][B] sum_{nu in B} x[nu]
-__global__ void atom_gamma_kernel(int n, int n_atoms, const int *ao_off, const int *ao_atom, const double *g,
-                                  const double *x1, const double *x2, double *xa1, double *xa2, double *gx1,
-                                  double *gx2) {
+// per-atom sums of two AO vectors and their gamma products:  out_ao[mu] = sum_B g[A(mu)][B] sum_{nu in B} x[nu];
+// one warp per atom, every CTA forms the atom sums
+__global__ void __launch_bounds__(256)
+atom_gamma_kernel(int n_atoms, const int *ao_off, const double *g, const double *x1, const double *x2, double *xa1,
+                  double *xa2, double *gx1, double *gx2) {
     extern __shared__ double sh[];
     double *s1 = sh, *s2 = sh + n_atoms;
     for (int A = threadIdx.x; A < n_atoms; A += blockDim.x) {
@@ -137,17 +136,25 @@ __global__ void atom_gamma_kernel(int n, int n_atoms, const int *ao_off, const i
         }
         s1[A] = a1;
         s2[A] = a2;
-        xa1[A] = a1;
-        xa2[A] = a2;
+        if (blockIdx.x == 0) {
+            xa1[A] = a1;
+            xa2[A] = a2;
+        }
     }
     __syncthreads();
-    for (int mu = threadIdx.x; mu < n; mu += blockDim.x) {
-        const double *gr = g + (long long)ao_atom[mu] * n_atoms;
-        double a1 = 0.0, a2 = 0.0;
-        for (int B = 0; B < n_atoms; ++B) {
-            a1 += gr[B] * s1[B];
-            a2 += gr[B] * s2[B];
-        }
+    const int A = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (A >= n_atoms) return;
+    const double *gr = g + (long long)A * n_atoms;
+    double a1 = 0.0, a2 = 0.0;
+    for (int B = lane; B < n_atoms; B += 32) {
+        a1 += gr[B] * s1[B];
+        a2 += gr[B] * s2[B];
+    }
+    for (int off = 16; off; off >>= 1) {
+        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, off);
+    }
+    for (int mu = ao_off[A] + lane; mu < ao_off[A + 1]; mu += 32) {
         gx1[mu] = a1;
         gx2[mu] = a2;
     }
@@ -195,57 +202,93 @@ __global__ void coulomb_p_kernel(int n, const int *ao_atom, const double *esp, c
     }
 }
 
-// single-block dot product
-__global__ void dot_kernel(long long len, const double *a, const double *b, double *out) {
-    __shared__ double red[32];
-    double s = 0.0;
-    for (long long x = threadIdx.x; x < len; x += blockDim.x) s += a[x] * b[x];
-    for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+// Device-side CG state: s[0] = r.r (r.z when preconditioned), s[1] = p.Ap, s[3] = beta; flag[0] = 0
+// while running, 1 once converged, 2 on a non-finite step; flag[1] = iterations done; flag[2] = CTAs of the
+// running reduction that are done.  Every thread forms alpha from the same two values, so all take the
+// same decision.
+
+// Sums of up to two values over the grid: every CTA leaves its part in part[blockIdx.x], the CTA that
+// is last adds the parts in CTA order (a fixed order) and returns true with the totals in its thread 0.
+__device__ bool cg_reduce(double a, double b, double2 *part, int *done, double &ta, double &tb) {
+    __shared__ double2 red[8];
+    __shared__ int last;
+    for (int off = 16; off; off >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, off);
+        b += __shfl_xor_sync(0xffffffffu, b, off);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(a, b);
     __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            a += red[w].x;
+            b += red[w].y;
+        }
+        part[blockIdx.x] = make_double2(a, b);
+        __threadfence();
+        last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    a = b = 0.0;
     if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-        if (threadIdx.x == 0) *out = s;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += 32) {
+            const double2 p = __ldcg(part + i);
+            a += p.x;
+            b += p.y;
+        }
+        for (int off = 16; off; off >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, off);
+            b += __shfl_xor_sync(0xffffffffu, b, off);
+        }
     }
+    if (threadIdx.x == 0) *done = 0;
+    ta = a;
+    tb = b;
+    return true;
 }
 
-// x += alpha p ; r -= alpha Ap
-__global__ void cg_update_kernel(long long len, double alpha, const double *p, const double *Ap, double *x, double *r) {
-    GRID_STRIDE(t, len) {
-        x[t] += alpha * p[t];
-        r[t] -= alpha * Ap[t];
-    }
+// *out = a.b
+__global__ void __launch_bounds__(256) cg_dot_kernel(long long len, const double *a, const double *b, double2 *part,
+                                                    int *flag, double *out) {
+    double s = 0.0, t, u;
+    GRID_STRIDE(x, len) s += a[x] * b[x];
+    if (cg_reduce(s, 0.0, part, flag + 2, t, u) && threadIdx.x == 0) *out = t;
 }
 
-// the same update with alpha = rr / pAp formed on the device (pAp left there by dot_kernel)
-// Device-side CG state: s[0] = r.r (r.z when preconditioned), s[1] = p.Ap, s[2] = the new r.r,
-// s[3] = beta, s[4] = the new r.z; flag[0] = 0 while running, 1 once converged, 2 on a non-finite
-// step; flag[1] = iterations done.  Every thread forms alpha from the same two values, so all take
-// the same decision.
-
-// x += alpha p ; r -= alpha Ap, alpha = r.r / p.Ap (skipped once the recursion has stopped)
-__global__ void cg_update_dev_kernel(long long len, const double *s, const int *flag, const double *p,
-                                     const double *Ap, double *x, double *r) {
+// One CG step: alpha = s[0] / s[1], x += alpha p, r -= alpha Ap, zr = r / omega when preconditioned (zr
+// not null), then the convergence test of helpers.rs:1146-1223 (r.r <= conv) and the next beta by the
+// CTA that finishes last.  Skipped once the recursion has stopped.
+__global__ void __launch_bounds__(256) cg_step_kernel(long long len, double *s, int *flag, double conv, const double *p,
+                                                     const double *Ap, const double *omega, double *x, double *r,
+                                                     double *zr, double2 *part) {
     if (flag[0] != 0) return;
     const double alpha = s[0] / s[1];
-    if (!isfinite(alpha)) return;   // cg_check_kernel records it
+    const bool fin = isfinite(alpha);
+    double rr = 0.0, rz = 0.0, trr, trz;
     GRID_STRIDE(t, len) {
-        x[t] += alpha * p[t];
-        r[t] -= alpha * Ap[t];
+        double rt = r[t];
+        if (fin) {
+            x[t] += alpha * p[t];
+            rt -= alpha * Ap[t];
+            r[t] = rt;
+        }
+        rr += rt * rt;
+        if (zr) {
+            const double z = rt / omega[t];
+            zr[t] = z;
+            rz += rt * z;
+        }
     }
-}
-
-// the convergence test of helpers.rs:1146-1223 (r.r <= conv) and the next beta
-__global__ void cg_check_kernel(double *s, int *flag, double conv, int precond) {
-    if (flag[0] != 0) return;
+    // every thread of the grid has read flag and s before its CTA counts itself done
+    if (!cg_reduce(rr, rz, part, flag + 2, trr, trz) || threadIdx.x != 0) return;
     flag[1] += 1;
-    if (!isfinite(s[0] / s[1])) {
+    if (!fin) {
         flag[0] = 2;
-    } else if (s[2] <= conv) {
+    } else if (trr <= conv) {
         flag[0] = 1;
     } else {
-        const double next = precond ? s[4] : s[2];
+        const double next = zr ? trz : trr;
         s[3] = next / s[0];
         s[0] = next;
     }
@@ -293,7 +336,64 @@ struct PairArgs {
     double *grad;                                // [3N] (written)
 };
 
-__global__ void __launch_bounds__(128) pair_gradient_kernel(PairArgs a) {
+// g += sum_pq w_pq d M_pq / d r for one pair's block of S or H0 (w = the adjoint's block at W, orbital p of
+// centre 1, q of centre 2; r = the vector from centre 1 to 2, u = r / |r|), summed over the block before
+// anything is differentiated: with w's s-s entry a, its s-p and p-s vectors b and c, its p-p matrix m,
+//     sum_pq w_pq M_pq = a V0 + (b.u) V1 + (c.u) V2 + (u m u) (V4 - V3) + tr(m) V3
+// in the integrals V of sk_element's slot order, whose gradient needs no angular factors per element.
+__device__ __forceinline__ void sk_contract(const PairArgs &a, int k1, int k2, int n1, int n2, const double *W,
+                                            const double *cf, const double N3[4], const double fd[3], const double u[3],
+                                            double r, double g[3]) {
+    double w[4][4] = {};   // rows and columns s, x, y, z
+    bool p1 = false, p2 = false;   // centres with p orbitals
+    for (int p = 0; p < n1; ++p) {
+        const int rp = a.kind_l[k1 * 4 + p] == 0 ? 0 : 1 + p_axis(a.kind_m[k1 * 4 + p]);
+        p1 = p1 || rp > 0;
+        for (int q = 0; q < n2; ++q) {
+            const int rq = a.kind_l[k2 * 4 + q] == 0 ? 0 : 1 + p_axis(a.kind_m[k2 * 4 + q]);
+            p2 = p2 || rq > 0;
+            w[rp][rq] += W[(long long)p * a.n_orb + q];
+        }
+    }
+    double v[SK_SLOTS], dv[SK_SLOTS];
+#pragma unroll
+    for (int s = 0; s < SK_SLOTS; ++s) {
+        const double *c = cf + (long long)s * a.n_knots;
+        const double c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+        v[s] = c0 * N3[0] + c1 * N3[1] + c2 * N3[2] + c3 * N3[3];
+        dv[s] = (c1 - c0) * fd[0] + (c2 - c1) * fd[1] + (c3 - c2) * fd[2];
+    }
+    double along = w[0][0] * dv[0], t[3] = {0.0, 0.0, 0.0};   // gradient along u; t: vectors to project
+    const double ri = 1.0 / r;
+    if (p2) {
+        const double bu = w[0][1] * u[0] + w[0][2] * u[1] + w[0][3] * u[2];
+        along += bu * (dv[1] - v[1] * ri);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] += w[0][1 + c] * v[1];
+    }
+    if (p1) {
+        const double cu = w[1][0] * u[0] + w[2][0] * u[1] + w[3][0] * u[2];
+        along += cu * (dv[2] - v[2] * ri);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] += w[1 + c][0] * v[2];
+    }
+    if (p1 && p2) {
+        const double D = v[4] - v[3], dD = dv[4] - dv[3];
+        double mu[3];   // (m + m^T) u
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            mu[c] = (w[1 + c][1] + w[1][1 + c]) * u[0] + (w[1 + c][2] + w[2][1 + c]) * u[1] + (w[1 + c][3] + w[3][1 + c]) * u[2];
+        const double umu2 = mu[0] * u[0] + mu[1] * u[1] + mu[2] * u[2];   // 2 u m u
+        along += 0.5 * umu2 * dD + (w[1][1] + w[2][2] + w[3][3]) * dv[3] - umu2 * D * ri;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] += mu[c] * D;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[c] += along * u[c] + t[c] * ri;
+}
+
+
+__global__ void __launch_bounds__(256) pair_gradient_kernel(PairArgs a) {
     const int i = blockIdx.x;
     const double xi = a.xyz[3 * i], yi = a.xyz[3 * i + 1], zi = a.xyz[3 * i + 2];
     const int ki = a.kind[i];
@@ -315,37 +415,23 @@ __global__ void __launch_bounds__(128) pair_gradient_kernel(PairArgs a) {
             double u[3] = {rv[0] / r, rv[1] / r, rv[2] / r};
             int l;
             double N3[4], N2[3];
-            double vS[SK_SLOTS] = {0, 0, 0, 0, 0}, dS[SK_SLOTS] = {0, 0, 0, 0, 0};
-            double vH[SK_SLOTS] = {0, 0, 0, 0, 0}, dH[SK_SLOTS] = {0, 0, 0, 0, 0};
             if (bspline3_basis(a.knots, a.n_knots, r, l, N3, N2, a.sk_extrapolate != 0)) {
-                const double *cS = a.coef + (long long)((k1 * a.n_kinds + k2) * 2 + 0) * SK_SLOTS * a.n_knots;
-                const double *cH = a.coef + (long long)((k1 * a.n_kinds + k2) * 2 + 1) * SK_SLOTS * a.n_knots;
-                for (int s = 0; s < SK_SLOTS; ++s) {
-                    bspline3_eval(a.knots, cS + (long long)s * a.n_knots, l, N3, N2, vS[s], dS[s]);
-                    bspline3_eval(a.knots, cH + (long long)s * a.n_knots, l, N3, N2, vH[s], dH[s]);
+                double fd[3];   // s'(r) = sum_j fd[j] (c_i - c_{i-1}), i = l - 2 + j
+                for (int q = 0; q < 3; ++q) {
+                    const double den = a.knots[l + 1 + q] - a.knots[l - 2 + q];
+                    fd[q] = den != 0.0 ? 3.0 / den * N2[q] : 0.0;
                 }
-            }
-            // d/dR_i = -d/dr when i is centre 1 (r = R_j - R_i), +d/dr otherwise
-            double sgn = c1_is_i ? -1.0 : 1.0;
-            int n1 = a.kind_norb[k1], n2 = a.kind_norb[k2];
-            int off1 = a.ao_off[c1], off2 = a.ao_off[c2];
-            for (int p = 0; p < n1; ++p) {
-                int lp = a.kind_l[k1 * 4 + p], mp = a.kind_m[k1 * 4 + p];
-                for (int q = 0; q < n2; ++q) {
-                    int lq = a.kind_l[k2 * 4 + q], mq = a.kind_m[k2 * 4 + q];
-                    long long idx = (long long)(off1 + p) * a.n_orb + (off2 + q);
-                    double val, gr[3];
-                    if (a.Ssym) {
-                        sk_element(lp, mp, lq, mq, u, r, vS, dS, val, gr);
-                        double w = sgn * a.Ssym[idx];
-                        g0 += w * gr[0]; g1 += w * gr[1]; g2 += w * gr[2];
-                    }
-                    if (a.Hsym) {
-                        sk_element(lp, mp, lq, mq, u, r, vH, dH, val, gr);
-                        double w = sgn * a.Hsym[idx];
-                        g0 += w * gr[0]; g1 += w * gr[1]; g2 += w * gr[2];
-                    }
-                }
+                const int n1 = a.kind_norb[k1], n2 = a.kind_norb[k2];
+                const long long at = (long long)a.ao_off[c1] * a.n_orb + a.ao_off[c2];
+                const double *cf = a.coef + (long long)((k1 * a.n_kinds + k2) * 2) * SK_SLOTS * a.n_knots + (l - 3);
+                double g[3] = {0.0, 0.0, 0.0};
+                if (a.Ssym) sk_contract(a, k1, k2, n1, n2, a.Ssym + at, cf, N3, fd, u, r, g);
+                if (a.Hsym) sk_contract(a, k1, k2, n1, n2, a.Hsym + at, cf + (long long)SK_SLOTS * a.n_knots, N3, fd, u, r, g);
+                // d/dR_i = -d/dr when i is centre 1 (r = R_j - R_i), +d/dr otherwise
+                const double sgn = c1_is_i ? -1.0 : 1.0;
+                g0 += sgn * g[0];
+                g1 += sgn * g[1];
+                g2 += sgn * g[2];
             }
         }
         // ---- gamma terms (gamma_approximation.rs:256-282, :392-423) ----
@@ -375,7 +461,7 @@ __global__ void __launch_bounds__(128) pair_gradient_kernel(PairArgs a) {
             }
         }
     }
-    __shared__ double red[3][4];
+    __shared__ double red[3][8];
     for (int off = 16; off; off >>= 1) {
         g0 += __shfl_down_sync(0xffffffffu, g0, off);
         g1 += __shfl_down_sync(0xffffffffu, g1, off);
@@ -507,9 +593,11 @@ void Ctx::pv_adjoint(const double *V, const double *Y, double scale, double *PS,
     const int n = n_orb;
     gv.reserve(4 * (size_t)n + 2 * (size_t)n_atoms);
     double *sv = gv.p, *r = sv + n, *gsv = r + n, *gr = gsv + n, *svA = gr + n, *rA = svA + n_atoms;
-    EW(fv_vectors_kernel, 2LL * n, n, dS_.p, V, Y, sv, r);
-    atom_gamma_kernel<<<1, 256, 2 * n_atoms * sizeof(double), stream>>>(n, n_atoms, d_ao_off.p, d_ao_atom.p, d_gamma.p,
-                                                                         sv, r, svA, rA, gsv, gr);
+    fv_vectors_kernel<<<ceil_div(2LL * n * 32, 256), 256, 0, stream>>>(n, dS_.p, V, Y, sv, r);
+    count_launch(stream, "fv_vectors");
+    check_launch("fv_vectors");
+    atom_gamma_kernel<<<ceil_div(n_atoms, 8), 256, 2 * n_atoms * sizeof(double), stream>>>(n_atoms, d_ao_off.p, d_gamma.p, sv,
+                                                                                           r, svA, rA, gsv, gr);
     count_launch(stream, "atom_gamma");
     check_launch("atom_gamma");
     EW(pv_accumulate_kernel, (long long)n * n, n, n_atoms, scale, V, Y, gsv, gr, PS);
@@ -520,8 +608,10 @@ void Ctx::pv_adjoint(const double *V, const double *Y, double scale, double *PS,
 // CG on (operator) Z = R  (helpers.rs:1130-1223): x0 = R / omega, stop when r.r <= conv.
 int Ctx::zvector_cg(int variant, const double *R, double *Z, int max_iter, double conv, int *iters) {
     const long long len = ov;
-    gcg.reserve(5 * (size_t)len + 8);
+    const int blocks = gridn(len, n_sm);   // of the reductions
+    gcg.reserve(5 * (size_t)len + 8 + 2 * (size_t)blocks + 1);
     double *r = gcg.p, *p = r + len, *Ap = p + len, *tmp = Ap + len, *Xt = tmp + len, *dots = Xt + len;
+    double2 *part = reinterpret_cast<double2 *>(dots + 8 + (5 * len) % 2);   // 16-byte aligned
     int h_flag[2] = {0, 0};
     auto op = [&](const double *x, double *out) {
         // tincr: TDA matrix A for LC (mult_av_lc: 2 Coulomb - exchange), A+B without exchange otherwise
@@ -532,11 +622,6 @@ int Ctx::zvector_cg(int variant, const double *R, double *Z, int max_iter, doubl
             EW(transpose_batched_kernel, len, 1, n_occ, n_virt, x, Xt);
             ao_contract(1, BLK_VIRT, BLK_OCC, Xt, BLK_OCC, BLK_VIRT, -0.25, 0.0, out, 1.0, 1.0, nullptr);
         }
-    };
-    auto dot_dev = [&](const double *a, const double *b, double *out) {   // out on the device, no sync
-        dot_kernel<<<1, 1024, 0, stream>>>(len, a, b, out);
-        count_launch(stream, "dot");
-        check_launch("dot");
     };
     EW(zguess_kernel, len, len, R, d_omega.p, Z);          // bs = R / omega
     int *flag = reinterpret_cast<int *>(dots + 6);
@@ -555,23 +640,15 @@ int Ctx::zvector_cg(int variant, const double *R, double *Z, int max_iter, doubl
         EW(axpby3_kernel, len, len, 1.0, R, -1.0, Ap, 0.0, nullptr, r);   // r = R - A Z
         if (pre) EW(zguess_kernel, len, len, r, d_omega.p, zr);
         TINCR_CUDA(cudaMemcpyAsync(p, dir, len * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-        dot_dev(r, dir, dots);
-        TINCR_CUDA(cudaMemsetAsync(flag, 0, 2 * sizeof(int), stream));
+        TINCR_CUDA(cudaMemsetAsync(flag, 0, 3 * sizeof(int), stream));
+        EW(cg_dot_kernel, len, len, r, dir, part, flag, dots);
         int queued = 0;
         while (queued < limit) {
             const int batch = std::min(CG_SYNC, limit - queued);
             for (int q = 0; q < batch; ++q) {
                 op(p, Ap);
-                dot_dev(p, Ap, dots + 1);
-                EW(cg_update_dev_kernel, len, len, dots, flag, p, Ap, Z, r);
-                dot_dev(r, r, dots + 2);
-                if (pre) {
-                    EW(zguess_kernel, len, len, r, d_omega.p, zr);
-                    dot_dev(r, zr, dots + 4);
-                }
-                cg_check_kernel<<<1, 1, 0, stream>>>(dots, flag, conv, pre ? 1 : 0);
-                count_launch(stream, "cg_check");
-                check_launch("cg_check");
+                EW(cg_dot_kernel, len, len, p, Ap, part, flag, dots + 1);
+                EW(cg_step_kernel, len, len, dots, flag, conv, p, Ap, d_omega.p, Z, r, pre ? zr : nullptr, part);
                 EW(cg_dir_kernel, len, len, dots, flag, p, dir);
             }
             queued += batch;
@@ -618,16 +695,26 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
     }
     const int n = n_orb, o = n_occ, v = n_virt, N = n_atoms;
     const size_t nn = (size_t)n * n;
+    // device temporaries: one slot per request, kept by the context (about 30 pairs of cudaMalloc and
+    // cudaFree on each call otherwise, each a device synchronisation)
+    size_t slot_no = 0;
+    struct Buf { double *p; };
+    auto take = [&](size_t count) {
+        if (slot_no == gtmp.size()) gtmp.emplace_back();
+        DevBuf<double> &d = gtmp[slot_no++];
+        d.reserve(std::max<size_t>(count, 1));
+        return Buf{d.p};
+    };
     g_launches = 0;
     prec = solve_prec;   // the contractions follow the precision the roots were solved with
     TINCR_CUDA(cudaEventRecord(ev0, stream));
-    DevBuf<int> dkind(N);
-    TINCR_CUDA(cudaMemcpyAsync(dkind.p, atom_kind, N * sizeof(int), cudaMemcpyHostToDevice, stream));
+    int *dkind = reinterpret_cast<int *>(take((N + 1) / 2).p);
+    TINCR_CUDA(cudaMemcpyAsync(dkind, atom_kind, N * sizeof(int), cudaMemcpyHostToDevice, stream));
     // dP = P - P0
     std::vector<double> hp0(n);
     for (int A = 0; A < N; ++A)
         for (int mu = h_ao_off[A]; mu < h_ao_off[A + 1]; ++mu) hp0[mu] = h_kind_occ[4 * atom_kind[A] + (mu - h_ao_off[A])];
-    DevBuf<double> dPm(nn), dDP(nn), dqd(N);
+    const Buf dPm = take(nn), dDP = take(nn), dqd = take(N);
     TINCR_CUDA(cudaMemcpyAsync(dPm.p, P, nn * sizeof(double), cudaMemcpyHostToDevice, stream));
     TINCR_CUDA(cudaMemcpyAsync(dqd.p, dq, N * sizeof(double), cudaMemcpyHostToDevice, stream));
     {
@@ -636,11 +723,12 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         TINCR_CUDA(cudaMemcpyAsync(dDP.p, dp.data(), nn * sizeof(double), cudaMemcpyHostToDevice, stream));
         sync();
     }
-    DevBuf<double> PS(nn), PH(nn), Ssym(nn), Hsym(nn), QG((size_t)N * N), QL((size_t)N * N), QGs((size_t)N * N),
-        QLs((size_t)N * N), dgrad(3 * (size_t)N);
+    const Buf PS = take(nn), PH = take(nn), Ssym = take(nn), Hsym = take(nn), QG = take((size_t)N * N),
+              QL = take((size_t)N * N), QGs = take((size_t)N * N), QLs = take((size_t)N * N),
+              dgrad = take(3 * (size_t)N);
     PairArgs pa{};
     pa.n_atoms = N; pa.n_orb = n; pa.n_kinds = n_kinds; pa.n_knots = n_knots;
-    pa.xyz = d_xyz.p; pa.kind = dkind.p; pa.ao_off = d_ao_off.p;
+    pa.xyz = d_xyz.p; pa.kind = dkind; pa.ao_off = d_ao_off.p;
     pa.kind_norb = d_kind_norb.p; pa.kind_l = d_kind_l.p; pa.kind_m = d_kind_m.p; pa.kind_z = d_kind_z.p;
     pa.sigma = d_sigma.p; pa.knots = d_knots.p; pa.coef = d_coef.p;
     pa.r_lr = r_lr_;
@@ -656,7 +744,7 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         pa.rep_ntmax = rep_ntmax; pa.rep_knots = d_rep_knots.p; pa.rep_coef = d_rep_coef.p; pa.rep_dmax = d_rep_dmax.p;
         pa.grad = dgrad.p;
         int slot = prof_begin(TINCR_KF_GRADIENT);
-        pair_gradient_kernel<<<N, 128, 0, stream>>>(pa);
+        pair_gradient_kernel<<<N, N > 128 ? 256 : 128, 0, stream>>>(pa);
         count_launch(stream, "pair_gradient");
         check_launch("pair_gradient");
         prof_end(slot, 0.0, 8.0 * (4.0 * nn + 4.0 * N * N));
@@ -685,7 +773,7 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         TINCR_CUDA(cudaMemsetAsync(QL.p, 0, (size_t)N * N * sizeof(double), stream));
         TINCR_CUDA(cudaMemcpyAsync(PH.p, dPm.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, stream));  // dH0 . P
         // - dS . W with W = 1/2 P H P
-        DevBuf<double> dH(nn), tmp(nn);
+        const Buf dH = take(nn), tmp = take(nn);
         TINCR_CUDA(cudaMemcpyAsync(dH.p, h_coul_x, nn * sizeof(double), cudaMemcpyHostToDevice, stream));
         mm(false, false, n, n, n, dPm.p, n, dH.p, n, tmp.p, n, 1.0, 0.0);
         mm(false, false, n, n, n, tmp.p, n, dPm.p, n, PS.p, n, -0.5, 1.0);
@@ -693,7 +781,7 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         std::vector<double> hdq(dq, dq + N), hg(h_gamma), esp(N, 0.0);
         for (int A = 0; A < N; ++A)
             for (int B = 0; B < N; ++B) esp[A] += hg[(size_t)A * N + B] * hdq[B];
-        DevBuf<double> desp(N);
+        const Buf desp = take(N);
         TINCR_CUDA(cudaMemcpyAsync(desp.p, esp.data(), N * sizeof(double), cudaMemcpyHostToDevice, stream));
         EW(coulomb_p_kernel, nn, n, d_ao_atom.p, desp.p, dPm.p, 1.0, PS.p);
         // + dq . dgamma . dq: QG = 1/2 dq dq^T so that the symmetrised block is dq_i dq_j
@@ -708,12 +796,13 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         const double omega_state = h_energies[state];
         const double *X = dR.p + (long long)state * ov;      // [o x v]
         std::vector<double> eo(h_orbe.begin(), h_orbe.begin() + o), ev(h_orbe.begin() + o, h_orbe.begin() + o + v);
-        DevBuf<double> deo(o), dev_(v);
+        const Buf deo = take(o), dev_ = take(v);
         TINCR_CUDA(cudaMemcpyAsync(deo.p, eo.data(), o * sizeof(double), cudaMemcpyHostToDevice, stream));
         TINCR_CUDA(cudaMemcpyAsync(dev_.p, ev.data(), v * sizeof(double), cudaMemcpyHostToDevice, stream));
         const size_t oo = (size_t)o * o, vv = (size_t)v * v;
-        DevBuf<double> Tij(oo), Tab(vv), Vij(oo), Vab(vv), tmpov(ov), gij(oo), qij(oo), qab(vv), hx(vv), qia(ov),
-            hq(oo), qai(ov), Rz(ov), Z(ov), wz(oo), Xt(ov);
+        const Buf Tij = take(oo), Tab = take(vv), Vij = take(oo), Vab = take(vv), tmpov = take(ov), gij = take(oo),
+                  qij = take(oo), qab = take(vv), hx = take(vv), qia = take(ov), hq = take(oo), qai = take(ov),
+                  Rz = take(ov), Z = take(ov), wz = take(oo), Xt = take(ov);
         mm(false, true, o, o, v, X, v, X, v, Tij.p, o, 1.0, 0.0);                 // X X^T
         mm(true, false, v, v, o, X, v, X, v, Tab.p, v, 1.0, 0.0);                 // X^T X
         EW(scale_rc_kernel, ov, o, v, X, nullptr, dev_.p, tmpov.p);             // X e_v
@@ -748,7 +837,8 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         }
         EW(axpby3_kernel, oo, (long long)oo, 1.0, qij.p, 1.0, wz.p, 0.0, nullptr, wz.p);
         const int m = o + v;
-        DevBuf<double> W((size_t)m * m), CW((size_t)n * m), Wao(nn), Mao(nn), Xao(nn), t1((size_t)n * std::max(o, v));
+        const Buf W = take((size_t)m * m), CW = take((size_t)n * m), Wao = take(nn), Mao = take(nn), Xao = take(nn),
+                  t1 = take((size_t)n * std::max(o, v));
         EW(w_assemble_kernel, (long long)m * m, o, v, wz.p, qai.p, Z.p, deo.p, qab.p, W.p);
         // W_AO = C triu(W) C^T   (C restricted to the o+v active MOs)
         mm(false, false, n, m, m, dC.p, n, W.p, m, CW.p, m, 1.0, 0.0);
@@ -772,7 +862,7 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         pv_adjoint(Xao.p, Xao.p, 0.5, PS.p, QG.p);
         if (lc) {
             plr_adjoint(dDP.p, Mao.p, -0.125, -0.125, PS.p, QL.p);
-            DevBuf<double> XaoT(nn);
+            const Buf XaoT = take(nn);
             EW(transpose_batched_kernel, nn, 1, n, n, Xao.p, XaoT.p);
             plr_adjoint(XaoT.p, Xao.p, -0.25, -0.25, PS.p, QL.p);
         }

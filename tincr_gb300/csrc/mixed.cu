@@ -207,6 +207,23 @@ void Ctx::qtrans_mixed(int k, const double *X, double *y_out) {
     if (use_tc) tc_err_watch();
 }
 
+// planes of A (M rows) and of B (N rows) in one launch (blockIdx.y picks the operand): [rows][kp] from
+// src[row][k], or src[k][row] when the operand's flag is set; columns K .. kp - 1 zero
+static __global__ void split_two_kernel(int M, int N, int K, const double *__restrict__ A, int lda, int at, bf16 *Ap,
+                                        const double *__restrict__ B, int ldb, int bt, bf16 *Bp, long long kp) {
+    const bool second = blockIdx.y != 0;
+    const double *src = second ? B : A;
+    const int ld = second ? ldb : lda, trans = second ? bt : at;
+    const long long total = (second ? N : M) * kp;
+    bf16 *dst = second ? Bp : Ap;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+        const int r = int(t / kp), c = int(t % kp);
+        float x = 0.f;
+        if (c < K) x = (float)(trans ? src[(long long)c * ld + r] : src[(long long)r * ld + c]);
+        store3(dst, total, t, x);
+    }
+}
+
 // C = alpha op(A) op(B) + beta C (row-major FP64 in and out) on the three-plane tensor-core GEMM:
 // op(A) is M x K (A[m*lda + k], or A[k*lda + m] when ta), op(B) is K x N (B[k*ldb + n], or
 // B[n*ldb + k] when tb).  The operands are split into planes per call (K padded to 64).
@@ -222,12 +239,10 @@ void Ctx::gemm_mixed(bool ta, bool tb, int M, int N, int K, const double *A, int
     }
     bf16 *Ap = mg_bf16.p, *Bp = Ap + N_PLANES * pa;
     // planes are written for every K column (padding included), so no memset is needed
-    split_planes_kernel<<<grid_of(pa, n_sm), 256, 0, stream>>>(1, M, K, A, lda, 0, ta ? 1 : 0, Ap, pa, kp, 0);
-    count_launch(stream, "split_planes");
-    check_launch("split_planes");
-    split_planes_kernel<<<grid_of(pb, n_sm), 256, 0, stream>>>(1, N, K, B, ldb, 0, tb ? 0 : 1, Bp, pb, kp, 0);
-    count_launch(stream, "split_planes");
-    check_launch("split_planes");
+    split_two_kernel<<<dim3(grid_of(std::max(pa, pb), n_sm), 2), 256, 0, stream>>>(M, N, K, A, lda, ta ? 1 : 0, Ap, B, ldb,
+                                                                                 tb ? 0 : 1, Bp, kp);
+    count_launch(stream, "split_two");
+    check_launch("split_two");
     plane_gemm(*this, TINCR_KF_GRADIENT, M, N, kp, PlaneOperand{Ap, pa, kp, 0}, PlaneOperand{Bp, pb, kp, 0}, 1,
                EpiPlaneOut{C, ldc, 0, nullptr, nullptr, alpha, beta}, K);
     if (use_tc) tc_err_watch();   // reported by the next sync()

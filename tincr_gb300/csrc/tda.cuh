@@ -97,6 +97,7 @@ struct Ctx {
     DevBuf<int> d_kind_z, d_kind_norb, d_kind_l, d_kind_m, d_rep_nt;
     DevBuf<double> d_sigma, d_knots, d_coef, d_rep_knots, d_rep_coef, d_rep_dmax;
     DevBuf<double> gw, gv, gcg;            // gradient workspaces
+    std::vector<DevBuf<double>> gtmp;      // its temporaries, by order of request
     int last_cg_status = TINCR_OK;
 
     int prec = TINCR_PREC_FP64;           // arithmetic of the contractions in ao_contract
