@@ -241,9 +241,13 @@ __global__ void ex_symmetrize_kernel(int n, double *H) {
 // A side-2 group (t, its monomers, the side-1 monomers) serves every s paired with it: the four LE
 // states of a monomer against one LE or CT state share V, which is formed once.
 
-// Per-monomer device views: C and S C ([n x n], row-major, columns = MOs), atom range, AO offsets.
+// What ex_vu_kernel<T> reads (orbitals, cross products, side rows, gamma_lr) is of type T: the FP32 form
+// reads FP32 copies made once per call, since a conversion from FP64 runs at the FP64 pipe's 2 per clock
+// and SM and every staged value took one (64 acenes: 19.8 ms with FP64 sources, 18.1 ms with FP32 ones).
+
+// Per-monomer device views: C and S C ([n x n] of T, row-major, columns = MOs), atom range, AO offsets.
 struct ExMono {
-    const double *C, *SC;
+    const void *C, *SC;
     const int *ao_off;   // [n_atoms + 1], local
     int n, n_atoms, atom0;
 };
@@ -254,8 +258,8 @@ struct ExS1 {
     int p0, np, q0, na;              // columns P of x1, Q of y1 (start), a extent
     const double *X1;                // b1(i, a) = X1[(i1 + i) * ld1 + a1 + a]
     int ld1, i1, a1;
-    const double *cross_yx1;         // S_y1x1 C_x1 [n_y1 x n_x1] (two monomers)
-    const double *cross_xy1;         // S_x1y1 C_y1 [n_x1 x n_y1] (two monomers)
+    const void *cross_yx1;           // S_y1x1 C_x1 [n_y1 x n_x1] (two monomers), of T
+    const void *cross_xy1;           // S_x1y1 C_y1 [n_x1 x n_y1] (two monomers)
     long long own;                   // rows of x1: L1c at own, L1s at own + n_x1 na, [mu][a] (per state)
     long long crs;                   // rows of y1: L1s at crs, [mu - n_x1][a] (per state and y1; L1c = 0)
 };
@@ -268,7 +272,7 @@ struct ExS2 {
     int ta, tj;                      // tile sides over a and j (ta tj <= XJ_T)
     const double *X2;                // b2(j, b) = X2[(j2 + j) * ld2 + b2 + b]
     int ld2, j2, b2;
-    const double *cross_xy2, *cross_yx2;
+    const void *cross_xy2, *cross_yx2;   // of T
     long long own;                   // rows of y2 (x2 = y2: all rows): R2c at own, R2s at own + n_y2 nq, [nu][j]
     long long crs;                   // rows of x2 when x2 != y2: R2s at crs, [nu][j] (per state and x2; R2c = 0)
 };
@@ -278,7 +282,9 @@ struct ExEl {
     int k1, k2;                      // side-1 and side-2 groups
 };
 
-constexpr int XJ_T = 128;            // threads per CTA: the largest (a, j) tile
+constexpr int XJ_T = 128;            // the largest (a, j) tile
+constexpr int XJ_G = 4;              // thread groups per tile, sharing out its atoms
+constexpr int XJ_TH = XJ_T * XJ_G;   // threads per CTA
 constexpr int XJ_TS = 16;            // largest tile side
 constexpr int XJ_AO = 2 * 102 + 4;   // AOs of two monomers (largest supported monomer: 102 AOs)
 constexpr int XJ_ATOMS = 80;         // atoms of two monomers (largest supported monomer: 40 atoms)
@@ -307,7 +313,7 @@ struct ExVUSmem {
     static constexpr size_t V_BYTES = sizeof(T) * XJ_ATOMS * XJ_T;
     static constexpr size_t END =
         W_BYTES + ST_BYTES > V_OFF + V_BYTES ? W_BYTES + ST_BYTES : V_OFF + V_BYTES;
-    static constexpr size_t BYTES = END + sizeof(double) * (XJ_T / 32);
+    static constexpr size_t BYTES = END + sizeof(double) * (XJ_TH / 32);
     static_assert(ST_BYTES <= V_OFF, "the side-1 staging of phase C would overlap V");
     static_assert(BYTES <= 227 * 1024, "over the shared memory of one CTA");
 };
@@ -315,12 +321,16 @@ struct ExVUSmem {
 // one CTA per (side-2 group, ta x tj tile of (a, j)):
 //   V^A_aj = sum_B gamma_lr[A, B] W^B_aj, then for every element (s, t) of the group
 //   H[s, t] -= sum_A sum_aj U^A_aj(s) V^A_aj
+// The kernel is bound by latency (L2 loads of the staging, dependent FMAs) at the two CTAs per SM that its
+// shared memory allows, so each tile has four groups of threads, which share out the staging, the atoms
+// B of W and the atom blocks A of V (U . V stays one sum over the atoms, of the first group): 64 acenes
+// in FP32 take 18.1 ms with one group, 13.9 with two, 13.0 with four.
 template <class T>
-__global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ tiles, const ExS2 *__restrict__ keys,
+__global__ void __launch_bounds__(XJ_TH) ex_vu_kernel(const int4 *__restrict__ tiles, const ExS2 *__restrict__ keys,
                                                      const int *__restrict__ el_begin, const ExEl *__restrict__ els,
                                                      const ExS1 *__restrict__ k1s, const ExMono *__restrict__ mono,
-                                                     const double *__restrict__ gamma_lr, int n_atoms_total,
-                                                     const double *__restrict__ scr, double *H, int n_states) {
+                                                     const T *__restrict__ gamma_lr, int n_atoms_total,
+                                                     const T *__restrict__ scr, double *H, int n_states) {
     constexpr int CH = sizeof(T) == 4 ? 16 : 8;   // atoms A per register block
     using L = ExVUSmem<T>;
     extern __shared__ __align__(16) unsigned char xv_raw[];
@@ -341,49 +351,50 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
     const bool two1 = K.x1 != K.y1, two2 = K.x2 != K.y2;
     const int nat1 = ex_nat(m1x, m1y, two1), nat2 = ex_nat(m2x, m2y, two2);
     const int nao1 = ex_nao(m1x, m1y, two1), nao2 = ex_nao(m2x, m2y, two2);
-    const int al = threadIdx.x / tj, jl = threadIdx.x % tj;
-    const bool active = threadIdx.x < ta * tj && a0 + al < K.na && j0 + jl < K.nq;
+    const int tt = threadIdx.x % XJ_T, grp = threadIdx.x / XJ_T;   // (a, j) of the tile; thread group
+    const int al = tt / tj, jl = tt % tj;
+    const bool active = tt < ta * tj && a0 + al < K.na && j0 + jl < K.nq;
 
     // ---- phase A: L2 = C_P', (S C)_P' (S_y2x2 C_x2 on y2) and R2 (side-2 scratch); W ----
 #pragma unroll 4
-    for (int e = threadIdx.x; e < nao2 * ta; e += XJ_T) {
+    for (int e = threadIdx.x; e < nao2 * ta; e += XJ_TH) {
         const int nu = e / ta, q = e % ta;
         T c = T(0), sc = T(0);
         if (a0 + q < K.na) {
             const int col = K.pa0 + a0 + q;
             if (nu < m2x.n) {
-                c = (T)m2x.C[(long long)nu * m2x.n + col];
-                sc = (T)m2x.SC[(long long)nu * m2x.n + col];
+                c = static_cast<const T *>(m2x.C)[(long long)nu * m2x.n + col];
+                sc = static_cast<const T *>(m2x.SC)[(long long)nu * m2x.n + col];
             } else {
-                sc = (T)K.cross_yx2[(long long)(nu - m2x.n) * m2x.n + col];
+                sc = static_cast<const T *>(K.cross_yx2)[(long long)(nu - m2x.n) * m2x.n + col];
             }
         }
         L2[nu][q] = T2{c, sc};
     }
     {
         const int ny2 = two2 ? m2y.n : m2x.n;   // rows held by the per-state part
-        const double *rc = scr + K.own, *rs = rc + (long long)ny2 * K.nq;
+        const T *rc = scr + K.own, *rs = rc + (long long)ny2 * K.nq;
 #pragma unroll 4
-        for (int e = threadIdx.x; e < nao2 * tj; e += XJ_T) {
+        for (int e = threadIdx.x; e < nao2 * tj; e += XJ_TH) {
             const int nu = e / tj, q = e % tj;
             T c = T(0), sc = T(0);
             if (j0 + q < K.nq) {
                 const int j = j0 + q;
                 if (!two2) {
-                    c = (T)rc[(long long)nu * K.nq + j];
-                    sc = (T)rs[(long long)nu * K.nq + j];
+                    c = rc[(long long)nu * K.nq + j];
+                    sc = rs[(long long)nu * K.nq + j];
                 } else if (nu < m2x.n) {
-                    sc = (T)scr[K.crs + (long long)nu * K.nq + j];
+                    sc = scr[K.crs + (long long)nu * K.nq + j];
                 } else {
-                    c = (T)rc[(long long)(nu - m2x.n) * K.nq + j];
-                    sc = (T)rs[(long long)(nu - m2x.n) * K.nq + j];
+                    c = rc[(long long)(nu - m2x.n) * K.nq + j];
+                    sc = rs[(long long)(nu - m2x.n) * K.nq + j];
                 }
             }
             R2[nu][q] = T2{c, sc};
         }
     }
     __syncthreads();
-    for (int B = 0; B < nat2; ++B) {
+    for (int B = grp; B < nat2; B += XJ_G) {
         const bool onx = B < m2x.n_atoms;
         const ExMono &mb = onx ? m2x : m2y;
         const int bl = onx ? B : B - m2x.n_atoms;
@@ -394,36 +405,36 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
                 const T2 l = L2[nu][al], r = R2[nu][jl];
                 w += l.x * r.y + l.y * r.x;
             }
-        W[B][threadIdx.x] = T(0.5) * w;
+        W[B][tt] = T(0.5) * w;
     }
     __syncthreads();   // the staged rows are dead: the gamma block takes their place
 
     // ---- phase B: gamma block, V = gamma W ----
     const int nA = (nat1 + CH - 1) / CH * CH;
 #pragma unroll 4
-    for (int e = threadIdx.x; e < nat2 * nA; e += XJ_T) {
+    for (int e = threadIdx.x; e < nat2 * nA; e += XJ_TH) {
         const int B = e / nA, A = e % nA;
         T g = T(0);
         if (A < nat1) {
             const int gA = A < m1x.n_atoms ? m1x.atom0 + A : m1y.atom0 + (A - m1x.n_atoms);
             const int gB = B < m2x.n_atoms ? m2x.atom0 + B : m2y.atom0 + (B - m2x.n_atoms);
-            g = (T)gamma_lr[(long long)gB * n_atoms_total + gA];   // gamma_lr is symmetric: A runs along a row
+            g = gamma_lr[(long long)gB * n_atoms_total + gA];   // gamma_lr is symmetric: A runs along a row
         }
         G[B][A] = g;
     }
     __syncthreads();
-    for (int A0 = 0; A0 < nat1; A0 += CH) {
+    for (int A0 = grp * CH; A0 < nat1; A0 += XJ_G * CH) {
         T acc[CH];
 #pragma unroll
         for (int k = 0; k < CH; ++k) acc[k] = T(0);
         for (int B = 0; B < nat2; ++B) {
-            const T w = W[B][threadIdx.x];
+            const T w = W[B][tt];
 #pragma unroll
             for (int k = 0; k < CH; ++k) acc[k] += G[B][A0 + k] * w;
         }
 #pragma unroll
         for (int k = 0; k < CH; ++k)
-            if (A0 + k < nat1) V[A0 + k][threadIdx.x] = acc[k];
+            if (A0 + k < nat1) V[A0 + k][tt] = acc[k];
     }
     __syncthreads();   // W and the gamma block are dead: the side-1 rows take their place
 
@@ -432,37 +443,37 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
     for (int ei = eb; ei < ee; ++ei) {
         const ExEl E = els[ei];
         const ExS1 K1 = k1s[E.k1];
-        const double *l1c = scr + K1.own, *l1s = l1c + (long long)m1x.n * K1.na;
+        const T *l1c = scr + K1.own, *l1s = l1c + (long long)m1x.n * K1.na;
 #pragma unroll 4
-        for (int e = threadIdx.x; e < nao1 * ta; e += XJ_T) {
+        for (int e = threadIdx.x; e < nao1 * ta; e += XJ_TH) {
             const int mu = e / ta, q = e % ta;
             T c = T(0), sc = T(0);
             if (a0 + q < K1.na) {
                 const int a = a0 + q;
                 if (mu < m1x.n) {
-                    c = (T)l1c[(long long)mu * K1.na + a];
-                    sc = (T)l1s[(long long)mu * K1.na + a];
+                    c = l1c[(long long)mu * K1.na + a];
+                    sc = l1s[(long long)mu * K1.na + a];
                 } else {
-                    sc = (T)scr[K1.crs + (long long)(mu - m1x.n) * K1.na + a];
+                    sc = scr[K1.crs + (long long)(mu - m1x.n) * K1.na + a];
                 }
             }
             L1[mu][q] = T2{c, sc};
         }
         if (ei == eb) {   // the same columns Q of y1 for every element of the group
 #pragma unroll 4
-            for (int e = threadIdx.x; e < nao1 * tj; e += XJ_T) {
+            for (int e = threadIdx.x; e < nao1 * tj; e += XJ_TH) {
                 const int mu = e / tj, q = e % tj;
                 T c = T(0), sc = T(0);
                 if (j0 + q < K.nq) {
                     const int col = K1.q0 + j0 + q;
                     if (!two1) {
-                        c = (T)m1x.C[(long long)mu * m1x.n + col];
-                        sc = (T)m1x.SC[(long long)mu * m1x.n + col];
+                        c = static_cast<const T *>(m1x.C)[(long long)mu * m1x.n + col];
+                        sc = static_cast<const T *>(m1x.SC)[(long long)mu * m1x.n + col];
                     } else if (mu < m1x.n) {
-                        sc = (T)K1.cross_xy1[(long long)mu * m1y.n + col];
+                        sc = static_cast<const T *>(K1.cross_xy1)[(long long)mu * m1y.n + col];
                     } else {
-                        c = (T)m1y.C[(long long)(mu - m1x.n) * m1y.n + col];
-                        sc = (T)m1y.SC[(long long)(mu - m1x.n) * m1y.n + col];
+                        c = static_cast<const T *>(m1y.C)[(long long)(mu - m1x.n) * m1y.n + col];
+                        sc = static_cast<const T *>(m1y.SC)[(long long)(mu - m1x.n) * m1y.n + col];
                     }
                 }
                 R1[mu][q] = T2{c, sc};
@@ -470,7 +481,7 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
         }
         __syncthreads();
         T acc = T(0);
-        if (active) {
+        if (grp == 0 && active) {   // one sum over the atoms, in order
             for (int A = 0; A < nat1; ++A) {
                 const bool onx = A < m1x.n_atoms;
                 const ExMono &ma = onx ? m1x : m1y;
@@ -481,13 +492,15 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
                     const T2 l = L1[mu][al], r = R1[mu][jl];
                     u += l.x * r.y + l.y * r.x;
                 }
-                acc += u * V[A][threadIdx.x];
+                acc += u * V[A][tt];
             }
             acc *= T(0.5);
         }
-        double d = (double)acc;
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = d;
+        if (grp == 0) {
+            double d = (double)acc;
+            for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = d;
+        }
         __syncthreads();   // also: the next element's staging overwrites L1 only after every thread is done
         if (threadIdx.x == 0) {
             double tot = 0.0;
@@ -495,6 +508,11 @@ __global__ void __launch_bounds__(XJ_T) ex_vu_kernel(const int4 *__restrict__ ti
             atomicAdd(H + (long long)E.s * n_states + E.t, -tot);
         }
     }
+}
+
+// FP32 copy
+__global__ void ex_float_kernel(long long n, const double *__restrict__ x, float *y) {
+    for (long long t = blockIdx.x * 256LL + threadIdx.x; t < n; t += gridDim.x * 256LL) y[t] = (float)x[t];
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -990,8 +1008,6 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
     std::vector<ExMono> hm(n_mono);
     for (int k = 0; k < n_mono; ++k)
         hm[k] = ExMono{dC.p + offC[k], dSC.p + offC[k], dAo.p + offAo[k], nao[k], mono[k].n_atoms, atom0[k]};
-    DevBuf<ExMono> dm;
-    upload_vec(stream, dm, hm);
     auto nao_of = [&](int x, int y) { return (long long)nao[x] + (x != y ? nao[y] : 0); };
     auto nat_of = [&](int x, int y) { return (long long)mono[x].n_atoms + (x != y ? mono[y].n_atoms : 0); };
     std::vector<ExS1> k1v;
@@ -1150,11 +1166,21 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
         }
     }
     for (auto &v : tab) std::vector<int>().swap(v);
+    // device data of the exchange pass, which runs on while the host packs the next stage's inputs
+    DevBuf<double> d1;
+    DevBuf<float> f32;
+    DevBuf<ExMono> dm;
+    DevBuf<ExS1> dk1;
+    DevBuf<ExS2> dk2;
+    DevBuf<ExEl> del;
+    DevBuf<int> deb;
+    DevBuf<int4> dvt;
+    std::vector<int> el_begin;
+    std::vector<int4> vt;
     auto run_exchange = [&](auto zero) {
         using T = decltype(zero);
         if (elv.empty()) return;
         // side arrays (FP64 scratch) by batched GEMMs
-        DevBuf<double> d1;
         d1.alloc(std::max<long long>(1, scr));
         TINCR_CUDA(cudaMemsetAsync(d1.p, 0, d1.n * sizeof(double), stream));
         for (const SideJob &J : sjobs) {
@@ -1181,9 +1207,47 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
             }
         }
         gb.run(*this, sizeof(T) == 4, dJobs, dTiles, TINCR_KF_AO_EXCHANGE);
+        // the T view of what ex_vu_kernel reads: the FP64 arrays themselves, or FP32 copies of them
+        const T *scr_t, *glr_t;
+        if constexpr (sizeof(T) == 4) {
+            const size_t nc = offC[n_mono], nx = dCross.n, n1 = d1.n;
+            f32.alloc(2 * nc + nx + n1 + n_g);
+            float *fC = f32.p, *fSC = fC + nc, *fX = fSC + nc, *f1 = fX + nx, *fG = f1 + n1;
+            auto copy = [&](size_t n, const double *x, float *y) {
+                ex_float_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 32u * n_sm), 256, 0, stream>>>((long long)n, x, y);
+                count_launch(stream, "ex_float");
+                check_launch("ex_float");
+            };
+            copy(nc, dC.p, fC);
+            copy(nc, dSC.p, fSC);
+            copy(nx, dCross.p, fX);
+            copy(n1, d1.p, f1);
+            copy(n_g, dGlr.p, fG);
+            auto moved = [&](const void *p) -> const void * {
+                return p ? fX + (static_cast<const double *>(p) - dCross.p) : nullptr;
+            };
+            for (int k = 0; k < n_mono; ++k) {
+                hm[k].C = fC + offC[k];
+                hm[k].SC = fSC + offC[k];
+            }
+            for (ExS1 &K : k1v) {
+                K.cross_yx1 = moved(K.cross_yx1);
+                K.cross_xy1 = moved(K.cross_xy1);
+            }
+            for (ExS2 &K : k2v) {
+                K.cross_xy2 = moved(K.cross_xy2);
+                K.cross_yx2 = moved(K.cross_yx2);
+            }
+            scr_t = f1;
+            glr_t = fG;
+        } else {
+            scr_t = d1.p;
+            glr_t = dGlr.p;
+        }
+        upload_vec(stream, dm, hm);
         // elements grouped by side-2 group (a stable counting sort); one CTA per (group, tile) forms V
         // and serves the group's elements
-        std::vector<int> el_begin(k2v.size() + 1, 0);
+        el_begin.assign(k2v.size() + 1, 0);
         for (const ExEl &E : elv) ++el_begin[E.k2 + 1];
         for (size_t k = 0; k < k2v.size(); ++k) el_begin[k + 1] += el_begin[k];
         {
@@ -1192,7 +1256,6 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
             for (const ExEl &E : elv) sorted[fill[E.k2]++] = E;
             elv.swap(sorted);
         }
-        std::vector<int4> vt;
         double fl = 0.0;
         for (int k = 0; k < (int)k2v.size(); ++k) {
             const ExS2 &K = k2v[k];
@@ -1202,11 +1265,6 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
             fl += (2.0 * nat_of(K.x1, K.y1) * nat_of(K.x2, K.y2) +
                    4.0 * nao_of(K.x1, K.y1) * (el_begin[k + 1] - el_begin[k])) * K.na * K.nq;
         }
-        DevBuf<ExS1> dk1;
-        DevBuf<ExS2> dk2;
-        DevBuf<ExEl> del;
-        DevBuf<int> deb;
-        DevBuf<int4> dvt;
         upload_vec(stream, dk1, k1v);
         upload_vec(stream, dk2, k2v);
         upload_vec(stream, del, elv);
@@ -1221,12 +1279,11 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
         const int slot = prof_begin(TINCR_KF_AO_EXCHANGE);
         for (size_t t0 = 0; t0 < vt.size(); t0 += 1u << 20) {   // grid limit
             const unsigned nb = (unsigned)std::min<size_t>(vt.size() - t0, 1u << 20);
-            ex_vu_kernel<T><<<nb, XJ_T, ExVUSmem<T>::BYTES, stream>>>(dvt.p + t0, dk2.p, deb.p, del.p, dk1.p, dm.p,
-                                                                       dGlr.p, n_atoms_total, d1.p, dH.p, ns);
+            ex_vu_kernel<T><<<nb, XJ_TH, ExVUSmem<T>::BYTES, stream>>>(dvt.p + t0, dk2.p, deb.p, del.p, dk1.p, dm.p,
+                                                                        glr_t, n_atoms_total, scr_t, dH.p, ns);
             count_launch(stream, "ex_vu");
             check_launch("ex_vu");
         }
-        sync();   // the host lists above must outlive their uploads
         prof_end(slot, fl, 0.0);
     };
     if (fp32)
