@@ -9,6 +9,9 @@
 //               32 x NB output block per CTA staged through shared memory, FP64 atomics into C.
 // skinny_comb:  Out[r][x] = epi(r, x, sum_i Y[r][i] V[i][x])   (r < R <= 32), one column per
 //               thread, Y staged in shared memory by 64-wide i chunks, coalesced reads of V rows.
+// Both are bound by the FP64 pipe of the SMs that have a CTA, so short vectors are cut finer: dots down
+// to 64 columns per CTA, combinations into CTAs of 64 columns x 4 rows (the sums over i keep their
+// order).  C20H22 (L = 2601, 10 roots): a dots call 164 -> 15 us, a combination 50 -> 20 us.
 #pragma once
 
 #include "common.cuh"
@@ -16,6 +19,7 @@
 namespace tincr {
 
 constexpr int SK_ROWS = 32, SK_COLS = 64, SK_T = 256;
+constexpr int SK_FULL = 152;   // SMs of a GB300
 
 // C[M x nb] += A[M x L] . B[nb x L]^T ; rows of B at or beyond nb are read as zero.
 template <int NB>
@@ -63,6 +67,7 @@ skinny_dots_guard_kernel(int M, int nb, int L, int l_chunk, const double *__rest
 
 // Out[r][x] = epi(r, x, sum_{i < m} Y(r, i) V[i][x]),  r < R (template, <= 32),
 // Y(r, i) = Y[r * ysr + i * ysi] (row-major [rows x m]: ysr = m, ysi = 1; transposed: ysr = 1, ysi = rows)
+// rows blockIdx.y R .. of Out per CTA
 template <int R, class Epi>
 __global__ void __launch_bounds__(SK_T)
 skinny_comb_kernel(int m, long long L, const double *__restrict__ Y, long long ysr, long long ysi,
@@ -71,16 +76,18 @@ skinny_comb_kernel(int m, long long L, const double *__restrict__ Y, long long y
     double acc[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = 0.0;
-    const long long x = blockIdx.x * (long long)SK_T + threadIdx.x;
+    const long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int r0 = blockIdx.y * R;
     for (int i0 = 0; i0 < m; i0 += 64) {
         const int ic = min(64, m - i0);
         __syncthreads();
-        for (int e = threadIdx.x; e < R * 64; e += SK_T) {
+        for (int e = threadIdx.x; e < R * 64; e += blockDim.x) {
             int r = e / 64, c = e % 64;
-            Ys[r][c] = (r < rows && c < ic) ? Y[(long long)r * ysr + (long long)(i0 + c) * ysi] : 0.0;
+            Ys[r][c] = (r0 + r < rows && c < ic) ? Y[(long long)(r0 + r) * ysr + (long long)(i0 + c) * ysi] : 0.0;
         }
         __syncthreads();
         if (x < L) {
+#pragma unroll 4
             for (int c = 0; c < ic; ++c) {
                 double v = V[(long long)(i0 + c) * ldv + x];
 #pragma unroll
@@ -91,7 +98,7 @@ skinny_comb_kernel(int m, long long L, const double *__restrict__ Y, long long y
     if (x < L)
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            if (r < rows) epi(r, x, acc[r]);
+            if (r0 + r < rows) epi(r0 + r, x, acc[r]);
 }
 
 // Epilogues of skinny_comb
@@ -123,7 +130,7 @@ inline void skinny_dots(cudaStream_t st, int n_sm, int M, int nb, long long L, c
     if (M <= 0 || nb <= 0 || L <= 0) return;
     int my = ceil_div(M, SK_ROWS);
     long long want = 2LL * n_sm;                       // CTAs in flight
-    long long chunks = std::max<long long>(1, std::min<long long>(want / my + 1, (L + 1023) / 1024));
+    long long chunks = std::max<long long>(1, std::min<long long>(want / my + 1, (L + SK_COLS - 1) / SK_COLS));
     int l_chunk = (int)(((L + chunks - 1) / chunks + SK_COLS - 1) / SK_COLS * SK_COLS);
     int gx = (int)((L + l_chunk - 1) / l_chunk);
     dim3 grid(gx, my);
@@ -141,6 +148,13 @@ template <class Epi>
 inline void skinny_comb(cudaStream_t st, int rows, int m, long long L, const double *Y, long long ysr, long long ysi,
                         const double *V, long long ldv, Epi epi) {
     if (rows <= 0 || L <= 0) return;
+    if ((L + SK_T - 1) / SK_T < SK_FULL) {   // fewer CTAs of 256 columns than SMs
+        skinny_comb_kernel<4, Epi><<<dim3((unsigned)((L + 63) / 64), (unsigned)((rows + 3) / 4)), 64, 0, st>>>(m, L, Y, ysr, ysi,
+                                                                                                         V, ldv, rows, epi);
+        count_launch(st, "skinny_comb");
+        check_launch("skinny_comb");
+        return;
+    }
     dim3 grid((unsigned)((L + SK_T - 1) / SK_T));
     // the FP64 pipe is the bound: rows are padded to the next multiple of 4 only
 #define TINCR_SKINNY_COMB(R) skinny_comb_kernel<R, Epi><<<grid, SK_T, 0, st>>>(m, L, Y, ysr, ysi, V, ldv, rows, epi)

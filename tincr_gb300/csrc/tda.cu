@@ -1011,6 +1011,9 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                 // then sequentially against the vectors accepted in this step (davidson.rs:162-168)
                 if (kadd <= 32 && coop_grid > 0) {
                     int slot = prof_begin(TINCR_KF_SUBSPACE);
+                    // no more CTAs than blocks of 256 elements: each barrier and each sum over the CTAs is
+                    // shorter, and empty CTAs only add zeros (C20H22, 10 corrections: 142 -> 132 us)
+                    const int gs_grid = (int)std::min<long long>(coop_grid, (ov + 255) / 256);
                     gs_part.reserve((size_t)2 * coop_grid * GS_SLOTS);
                     gs_state.reserve(2);
                     int hstate[2] = {m, 0};
@@ -1020,7 +1023,7 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                     double *a_V = dV.p, *a_T = dT.p, *a_part = gs_part.p;
                     int *a_state = gs_state.p;
                     void *args[] = {&a_kadd, &a_ov, &a_m0, &a_mmax, &a_V, &a_T, &a_part, &a_state};
-                    TINCR_CUDA(cudaLaunchCooperativeKernel((const void *)seq_gs_kernel, dim3(coop_grid), dim3(256), args,
+                    TINCR_CUDA(cudaLaunchCooperativeKernel((const void *)seq_gs_kernel, dim3(gs_grid), dim3(256), args,
                                                            0, stream));
                     count_launch(stream, "seq_gs");
                     prof_end(slot, 4.0 * kadd * (double)kadd * ov / 2.0, 8.0 * (kadd * (kadd + 3.0) / 2.0) * ov);
