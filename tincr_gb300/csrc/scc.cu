@@ -14,21 +14,26 @@
 // A cluster keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and
 // runs every step itself; its CTAs share out the tiles, rows, roots and elements of a step and meet at
 // the cluster barrier, small vectors and sums going straight into each other's shared memory:
-//  * GEMMs on tiles of 16 x 16 outputs, one per thread (FP64) or 32 x 32, 2 x 2 per thread (FP32).
-//    GB300 issues 2 FP64 FMAs per SM and clock against 128 FP32 FMAs, so the FP64 GEMMs are bound by
-//    the FP64 pipe and small tiles keep the padding of n = 48..256 matrices small;
+//  * the FP64 products of the iterations as exact digit products on warp MMAs (sc_prod); those of small
+//    systems, of the set-up and of the FP32 phase on tiles of 16 x 16 outputs, one per thread (FP64), or
+//    32 x 32, 2 x 2 per thread (FP32).  GB300 issues 2 FP64 FMAs per SM and clock, 1/64 of its FP32 rate;
+//  * the density of an iteration by purification (sc_purify), the eigenpairs of S and of the last Fock
+//    matrix (and of one without a gap) by a tridiagonal eigensolver;
 //  * eigenpairs: Householder tridiagonalisation, Sturm-count multisection (the lanes that the roots
 //    leave idle take more points per root), inverse iteration with one thread per root (LU with partial
-//    pivoting), Gram-Schmidt inside clusters of close roots (LAPACK dstein's criterion, 1e-3 of the
-//    tridiagonal's norm), and the back-transformation by the stored reflections;
+//    pivoting), Loewdin's orthogonalisation to first order (Gram-Schmidt inside clusters of close roots
+//    where that does not do), and the back-transformation by the stored reflections;
 //  * the Fock build, Mulliken charges, DIIS and the energy as element loops and reductions.
-// CTAs per system: the largest power of two up to 16 that keeps the batch within SC_FILL CTAs per SM.
-// One CTA per system left most SMs idle on small batches and ended every batch with its slowest
-// system.  Measured, one CTA per system / the rule (ms of the kernel, LC, to 1e-10): one decacene
-// (192 orbitals, 16 CTAs) 705 / 123, 16 acene dimers (up to 186 orbitals) 690 / 160, 40 dimers 719 / 233,
-// 75 dimers 728 / 367, 128 dimers 750 / 417, 64 acenes 145 / 74, 400 dimers (1 CTA each) 1100 / 1081.
-// With 2 or 8 CTAs per SM instead of 4, 128 dimers take 600 / 561.  What bounds it: the FP64 pipe in the
-// GEMMs (40 % of a system's time at 4 CTAs), the FP64 latency chains of the eigensolver otherwise.
+// CTAs per system: the largest power of two from 2 to 16 that keeps the batch within SC_FILL CTAs per SM.
+// Kernel time (ms, LC, to 1e-10) with one CTA per system, FP64 tiles and the eigensolver in every
+// iteration / with clusters / with digit products and purification too:
+//     one decacene (192 orbitals)  705 / 123 / 44       128 acene dimers (up to 186)  750 / 417 / 176
+//     16 acene dimers              690 / 160 / 54       64 acenes (up to 102)         145 /  74 /  37
+//     40 acene dimers              719 / 233 / 79       400 acene dimers             1100 / 1081 / 512
+// SC_FILL 2, 4 and 8: 40 dimers 109, 79, 123; 128 dimers 237, 176, 207; 200 dimers 438, 266, 261.  Below
+// SC_DIGITS the operand splits and barriers cost more than the FP64 tiles: 66 orbitals on 16 CTAs 10.2 ms
+// on tiles, 13.0 on digits.  What bounds it: the latency of the digit products' loads and barriers at
+// 16 CTAs per system, the tensor and integer pipes (digit splits) of full batches.
 // With TINCR_SCC_FP32_START the iterations run in FP32 until the commutator is below 1e-5 (at most
 // 60 of them), then continue in FP64 from that density with a fresh DIIS history: the stationary
 // point, the convergence test and the final orbitals are FP64 either way.
@@ -44,6 +49,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "fixed8.cuh"
 #include "sk_math.cuh"
 #include "tda.cuh"
 
@@ -61,6 +67,7 @@ constexpr double SC_FP32_SWITCH = 1e-5;
 constexpr double SC_PROXIMITY = 30.0;  // bohr: Slater-Koster pairs farther apart are zero (tincr's PROXIMITY_CUTOFF)
 constexpr int SC_SLOTS_PER_SM = 2;
 constexpr int SC_KS = 32;              // k depth of a GEMM slice
+constexpr int SC_DIGITS = 20000;       // n^3 per CTA from which the iterations' FP64 products run on digits
 constexpr int SC_CMAX = 16;            // CTAs per cluster
 constexpr int SC_FILL = 4;             // CTAs per SM that a batch is spread over (twice those that run at once)
 
@@ -295,6 +302,185 @@ __device__ __forceinline__ void gemm_sym(int M, int K, T alpha, const T *A, int 
 }
 
 // ---------------------------------------------------------------------------------------------
+// FP64 products of the iterations on the tensor cores
+// ---------------------------------------------------------------------------------------------
+//
+// The same exact digit products as the FP64 contraction's (fixed8.cuh), on warp MMAs, so that a CTA keeps
+// its registers and shared memory for the other steps: a warp computes its outputs from operands in
+// digit planes, which the split writes in the order of the MMA's fragments.  An operand's rows r and its K
+// elements are cut into 16 x 16 tiles (rt, kt); plane p of a tile is 32 x 16 bytes at
+// [((rt nkt + kt) 8 + p) 32 + lane], lane (g, t) = (lane / 4, lane % 4) holding
+// x: (row g, k 2t, 2t + 1), y: (row g, k 2t + 8, 2t + 9), z, w: the same of row g + 8: the registers of an A
+// fragment of m16n8k16, and with {x, y} and {z, w} those of two B fragments, so one form serves both
+// sides.  A warp's tile is 16 x 8, which leaves it the registers to have all loads of a 16-k block in
+// flight; its 32 level accumulators are exact over 128 k, then folded to FP64.
+
+// the eight planes of a lane's fixed-point values x, x, y, y, z, z, w, w
+__device__ __forceinline__ void sc_store(uint4 *d, const unsigned long long (&y)[8]) {
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+        d[p * 32] = make_uint4(cd_pair(y[0], y[1], p), cd_pair(y[2], y[3], p), cd_pair(y[4], y[5], p), cd_pair(y[6], y[7], p));
+}
+
+// digits of rows r < rows of K elements, element (r, k) at A[r * lda + k], or A[k * lda + r] when trans
+__device__ __noinline__ void sc_split(const double *A, int lda, bool trans, int rows, int K, uint4 *D, int *E, const ScShared &sm) {
+    const int lane = threadIdx.x & 31, nrt = (rows + 15) / 16, nkt = (K + 15) / 16;
+    const int warps = SC_W * sm.csize, parts = max(1, min(warps / nrt, nkt));   // warps per row tile
+    const int g = lane >> 2, t = lane & 3;
+    for (int task = sm.rank * SC_W + (threadIdx.x >> 5); task < nrt * parts; task += warps) {
+        const int rt = task % nrt, part = task / nrt, r0 = rt * 16;
+        // bound exponents of the tile's rows, lane r: row r0 + r
+        unsigned mx = 0;
+        if (trans) {
+            const int r = r0 + (lane & 15);
+            if (r < rows)
+#pragma unroll 4
+                for (int k = lane >> 4; k < K; k += 2) mx = max(mx, cd_hi(A[(long long)k * lda + r]));
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        } else {
+            for (int r = 0; r < 16; ++r) {
+                unsigned m = 0;
+                if (r0 + r < rows)
+#pragma unroll 4
+                    for (int k = lane; k < K; k += 32) m = max(m, cd_hi(A[(long long)(r0 + r) * lda + k]));
+                m = __reduce_max_sync(0xffffffffu, m);
+                if (lane == r) mx = m;
+            }
+        }
+        const int e = cd_bound(mx);
+        if (part == 0 && lane < 16) E[r0 + lane] = e;
+        const int e0 = __shfl_sync(0xffffffffu, e, g), e1 = __shfl_sync(0xffffffffu, e, g + 8);
+        for (int kt = part; kt < nkt; kt += parts) {
+            unsigned long long y[8];   // x, x, y, y, z, z, w, w
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r = r0 + g + (q >> 2) * 8, k = kt * 16 + 2 * t + ((q >> 1) & 1) * 8 + (q & 1);
+                const int ex = (q >> 2) ? e1 : e0;
+                const double v = r < rows && k < K && ex != CD_POISON
+                                     ? (trans ? A[(long long)k * lda + r] : A[(long long)r * lda + k]) : 0.0;
+                y[q] = cd_fixed(v, ex);
+            }
+            sc_store(D + ((long long)(rt * nkt + kt) * 8) * 32 + lane, y);
+        }
+    }
+}
+
+__device__ __forceinline__ void sc_mma(float (&c)[4], const uint4 &a, const uint2 &b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a.x), "r"(a.z), "r"(a.y), "r"(a.w), "r"(b.x), "r"(b.y));
+}
+
+// C = alpha A B^T + beta C from digits (A: M rows, B: N rows, K elements); `sym`: the tiles on and below
+// the diagonal are computed and mirrored.  Returns the calling thread's part of the trace of C.
+__device__ __noinline__ double sc_digit_gemm(int M, int N, int K, double alpha, const uint4 *A, const int *Ea, const uint4 *B,
+                                const int *Eb, double beta, double *C, int ldc, bool sym, const ScShared &sm) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nti = (M + 15) / 16, ntj = (N + 7) / 8, nkt = (K + 15) / 16;
+    const int count = sym ? nti * (nti + 1) : nti * ntj;   // sym: 2 (i + 1) column tiles in row tile i
+    double trace = 0.0;
+    for (int id = sm.rank * SC_W + (threadIdx.x >> 5); id < count; id += SC_W * sm.csize) {
+        int ti = id / ntj, tj = id % ntj;
+        if (sym) {
+            ti = (int)((sqrtf(4.0f * id + 1.0f) - 1.0f) * 0.5f);
+            while (ti * (ti + 1) > id) --ti;
+            while ((ti + 1) * (ti + 2) <= id) ++ti;
+            tj = id - ti * (ti + 1);
+            if (tj >= ntj) continue;
+        }
+        const int e0 = Ea[ti * 16 + g], e1 = Ea[ti * 16 + g + 8];
+        double out[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int kc = 0; kc < nkt; kc += 8) {
+            float acc[8][4];   // level, fragment
+#pragma unroll
+            for (int l = 0; l < 8; ++l)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[l][q] = 0.0f;
+            const int kend = min(kc + 8, nkt);
+#pragma unroll 1
+            for (int kt = kc; kt < kend; ++kt) {
+                const uint4 *pa = A + ((long long)(ti * nkt + kt) * 8) * 32 + lane;
+                const uint2 *pb = reinterpret_cast<const uint2 *>(B + ((long long)((tj >> 1) * nkt + kt) * 8) * 32 + lane) + (tj & 1);
+                uint4 a[8];
+                uint2 b[8];
+#pragma unroll
+                for (int p = 0; p < 8; ++p) {
+                    a[p] = pa[p * 32];
+                    b[p] = pb[p * 64];
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+#pragma unroll
+                    for (int p = 0; p < 8 - s; ++p) sc_mma(acc[s + p], a[s], b[p]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                auto lv = [&](int l) { return (long long)__float2int_rz(acc[l][q]); };
+                const long long Hs = (((lv(0) << 8) + lv(1)) << 16) + (lv(2) << 8) + lv(3);
+                const long long Ls = (((lv(4) << 8) + lv(5)) << 16) + (lv(6) << 8) + lv(7);
+                const int a_e = q >> 1 ? e1 : e0, b_e = Eb[tj * 8 + 2 * t + (q & 1)];
+                out[q] += a_e == CD_POISON || b_e == CD_POISON ? __longlong_as_double(0x7ff8000000000000ll)
+                                                               : cd_value(Hs, Ls, a_e + b_e - 68);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int m = ti * 16 + g + (q >> 1) * 8, n = tj * 8 + 2 * t + (q & 1);
+            if (m < M && n < N && !(sym && n > m)) {
+                double *c = C + (long long)m * ldc + n;
+                const double v = beta == 0.0 ? alpha * out[q] : fma(alpha, out[q], beta * *c);
+                *c = v;
+                if (sym && n < m) C[(long long)n * ldc + m] = v;
+                if (n == m) trace += v;
+            }
+        }
+    }
+    return trace;
+}
+
+// digit operands of a system: S and X (cut once), and the two of the running product
+struct ScDig {
+    uint4 *S, *X, *a, *b;
+    int *eS, *eX, *ea, *eb;
+};
+enum ScOp { OP_S, OP_X, OP_ANY };
+
+// whether the FP64 products of a system of n orbitals run on digits
+__device__ __forceinline__ bool sc_digits(int n, const ScShared &sm) { return n * n * n >= SC_DIGITS * sm.csize; }
+
+// A product of the iterations, C = alpha A B + beta C (A, B transposed when ta, tb): FP32 on tiles
+__device__ __forceinline__ void sc_prod(const ScDig &, int M, int N, int K, float alpha, ScOp, const float *A, int lda,
+                                        bool ta, ScOp, const float *B, int ldb, bool tb, float beta, float *C, int ldc,
+                                        bool sym, ScShared &sm) {
+    sc_gemm<float, ScTile<float>::R>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, sm, sym);
+}
+// ... FP64 on digits, or on FP64 tiles in small systems
+__device__ __noinline__ void sc_prod(const ScDig &dg, int M, int N, int K, double alpha, ScOp oa, const double *A, int lda,
+                                     bool ta, ScOp ob, const double *B, int ldb, bool tb, double beta, double *C, int ldc,
+                                     bool sym, ScShared &sm) {
+    if (!sc_digits(max(M, K), sm)) {
+        sc_gemm<double, ScTile<double>::R>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, sm, sym);
+        return;
+    }
+    const uint4 *da = oa == OP_S ? dg.S : oa == OP_X ? dg.X : dg.a, *db = ob == OP_S ? dg.S : ob == OP_X ? dg.X : dg.b;
+    const int *ea = oa == OP_S ? dg.eS : oa == OP_X ? dg.eX : dg.ea, *eb = ob == OP_S ? dg.eS : ob == OP_X ? dg.eX : dg.eb;
+    if (oa == OP_ANY) sc_split(A, lda, ta, M, K, dg.a, dg.ea, sm);
+    if (ob == OP_ANY) {
+        if (A == B && ta != tb) {   // A A^T or A^T A
+            db = da;
+            eb = ea;
+        } else {
+            sc_split(B, ldb, !tb, N, K, dg.b, dg.eb, sm);
+        }
+    }
+    sc_bar(sm);
+    sc_digit_gemm(M, N, K, alpha, da, ea, db, eb, beta, C, ldc, sym, sm);
+    sc_bar(sm);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Symmetric eigenproblem
 // ---------------------------------------------------------------------------------------------
 
@@ -368,7 +554,7 @@ __device__ __forceinline__ int sc_sturm(const float *d, const float *esq, int n,
 // next pivot row sends that row; after it each forms the updated pivot row (and so the next
 // reflection) itself.
 template <class T>
-__device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, ScShared &sm) {
+__device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, const ScDig &dg, ScShared &sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cs = sm.csize, rank = sm.rank;
     T *d = reinterpret_cast<T *>(sm.d), *e = reinterpret_cast<T *>(sm.e), *beta = reinterpret_cast<T *>(sm.beta);
     T *esq = reinterpret_cast<T *>(sm.esq), *u = reinterpret_cast<T *>(sm.vu), *cur = reinterpret_cast<T *>(sm.cur);
@@ -584,8 +770,26 @@ __device__ bool sc_eigh(int n, int nr, T *A, T *Z, T *ws, unsigned char *piv, Sc
 #undef IX
     }
     sc_bar(sm);
-    // 5. Gram-Schmidt (twice) inside clusters of roots closer than 1e-3 |T|, one warp per cluster
-    {
+    // 5. orthonormalisation.  Inverse iteration leaves overlaps of order eps |T| / gap, so Z^T Z = I + D with
+    //    a tiny D unless roots (nearly) coincide, and Z (I - D / 2) is orthonormal to D^2 (Loewdin's
+    //    orthogonalisation to first order): two products instead of a chain of Gram-Schmidt steps along
+    //    clusters that take in most of the spectrum at LAPACK dstein's 1e-3 |T|.  With overlaps of 1e-8 and
+    //    more: Gram-Schmidt (twice) inside clusters of roots closer than 1e-3 |T|, one warp per cluster.
+    T *D = ws, *Z2 = ws + (long long)nr * nr;
+    sc_prod(dg, nr, nr, n, T(1), OP_ANY, Z, nr, true, OP_ANY, Z, nr, false, T(0), D, nr, true, sm);
+    double dmax = 0.0;
+    SC_FOR(t, (long long)nr * nr) {
+        const int i = (int)(t / nr), j = (int)(t - (long long)i * nr);
+        const T v = (i == j ? T(1) : T(0)) - D[t];
+        dmax = fmax(dmax, fabs((double)v));
+        D[t] = T(0.5) * v;
+    }
+    dmax = sc_max(dmax, sm);
+    if (dmax < (sizeof(T) == 8 ? 1e-8 : 1e-4)) {
+        sc_bar(sm);
+        sc_prod(dg, n, nr, nr, T(1), OP_ANY, Z, nr, false, OP_ANY, D, nr, false, T(0), Z2, nr, false, sm);
+        SC_FOR(t, (long long)n * nr) Z[t] += Z2[t];
+    } else {
         const double ortol = 1e-3 * tnorm;
         int c0 = 0, id = 0;
         for (int r = 1; r < nr; ++r) {
@@ -716,12 +920,18 @@ struct ScSlot {
     double *S, *H0, *X, *Sh, *gam, *glr, *p0;
     unsigned char *work;
     unsigned char *piv;
+    ScDig dg;
 };
 
 constexpr int SC_WORK = 29;   // n x n blocks of the work area
 
 __host__ __device__ inline long long sc_slot_doubles(long long nn, long long at2, long long npad) {
     return 4 * nn + 2 * at2 + npad + SC_WORK * nn;
+}
+
+// bytes of the digit operands of a slot for np (a multiple of 16) orbitals, a multiple of 256
+__host__ __device__ inline long long sc_digit_bytes(long long np) {
+    return (4 * np * np * 16 + 4 * np * 4 + 255) / 256 * 256;
 }
 
 __device__ ScSlot sc_slot(const ScArgs &a, int slot) {
@@ -736,6 +946,18 @@ __device__ ScSlot sc_slot(const ScArgs &a, int slot) {
     s.p0 = s.glr + a.at2_max;
     s.work = reinterpret_cast<unsigned char *>(s.p0 + a.npad);
     s.piv = s.work + SC_WORK * a.nn_max * (long long)sizeof(double);
+    // digit planes (16-byte aligned): 16 bytes per element of 16 x 16 tiles, then the rows' exponents
+    const long long np = (a.npad + 15) / 16 * 16, per = np * np;
+    uint4 *d = reinterpret_cast<uint4 *>(a.ws + (long long)(slot + 1) * a.slot_bytes - sc_digit_bytes(np));
+    s.dg.S = d;
+    s.dg.X = d + per;
+    s.dg.a = d + 2 * per;
+    s.dg.b = d + 3 * per;
+    int *e = reinterpret_cast<int *>(d + 4 * per);
+    s.dg.eS = e;
+    s.dg.eX = e + np;
+    s.dg.ea = e + 2 * np;
+    s.dg.eb = e + 3 * np;
     return s;
 }
 
@@ -743,6 +965,7 @@ template <class T> struct ScWork {
     T *S, *H0, *X, *Sh, *gam, *glr;     // inputs in T (FP64: the slot's arrays)
     T *F, *Fp, *P, *Pp, *T1, *T2, *T3, *EA, *Z, *W;   // n x n each (W: 4 n x n)
     T *Fh, *Eh;                         // SC_DIIS n x n each
+    ScDig dg;
 };
 
 template <class T>
@@ -752,6 +975,7 @@ __device__ ScWork<T> sc_work(const ScSlot &s, long long nn) {
     w.F = b; w.Fp = b + nn; w.P = b + 2 * nn; w.Pp = b + 3 * nn; w.T1 = b + 4 * nn; w.T2 = b + 5 * nn;
     w.T3 = b + 6 * nn; w.EA = b + 7 * nn; w.Z = b + 8 * nn; w.W = b + 9 * nn;
     w.Fh = b + 13 * nn; w.Eh = b + (13 + SC_DIIS) * nn;
+    w.dg = s.dg;
     return w;
 }
 
@@ -920,14 +1144,14 @@ __device__ void sc_fock(int n, int N, bool lc, const ScWork<T> &w, const double 
     }
     sc_bar(sm);
 #define GLR(mu, nu) w.glr[(long long)sm.ao_atom[mu] * N + sm.ao_atom[nu]]
-    gemm<T>(n, n, n, T(1), w.S, n, false, dP, n, false, T(0), w.T1, n, sm);   // S dP
+    sc_prod(w.dg, n, n, n, T(1), OP_S, w.S, n, false, OP_ANY, dP, n, false, T(0), w.T1, n, false, sm);   // S dP
     SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         tmp[t] = GLR(mu, nu) * w.T1[t];
     }
     sc_bar(sm);
-    gemm<T>(n, n, n, T(1), tmp, n, false, w.S, n, false, T(0), w.T2, n, sm);   // (g o S dP) S
-    gemm_sym<T>(n, n, T(1), w.T1, n, false, w.S, n, false, T(0), w.T3, n, sm);   // S dP S
+    sc_prod(w.dg, n, n, n, T(1), OP_ANY, tmp, n, false, OP_S, w.S, n, false, T(0), w.T2, n, false, sm);   // (g o S dP) S
+    sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.T1, n, false, OP_S, w.S, n, false, T(0), w.T3, n, true, sm);   // S dP S
     SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         const T g = GLR(mu, nu);
@@ -935,8 +1159,8 @@ __device__ void sc_fock(int n, int N, bool lc, const ScWork<T> &w, const double 
         tmp[t] = dP[t] * g;
     }
     sc_bar(sm);
-    gemm<T>(n, n, n, T(1), w.S, n, false, tmp, n, false, T(0), w.T1, n, sm);   // S (dP o g)
-    gemm_sym<T>(n, n, T(1), w.T1, n, false, w.S, n, false, T(1), hx, n, sm);    // + S (dP o g) S
+    sc_prod(w.dg, n, n, n, T(1), OP_S, w.S, n, false, OP_ANY, tmp, n, false, T(0), w.T1, n, false, sm);   // S (dP o g)
+    sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.T1, n, false, OP_S, w.S, n, false, T(1), hx, n, true, sm);    // + S (dP o g) S
     SC_FOR(t, nn) {
         const int mu = (int)(t / n), nu = (int)(t - (long long)mu * n);
         w.F[t] += T(-0.0625) * (hx[t] + hx[(long long)nu * n + mu]);
@@ -981,6 +1205,85 @@ __device__ void sc_diis_solve(int m, int cur, ScShared &sm) {
     __syncthreads();
 }
 
+// Density of the o lowest states of the symmetric matrix F without its eigenpairs: X ends as the projector
+// onto them.  Trace-correcting purification (Niklasson, Phys. Rev. B 66, 155115 (2002)): X_0 maps the
+// spectrum into [0, 1] with the lowest states near 1, and each step takes X^2 or 2 X - X^2, whichever
+// brings the trace closer to o, until X = X^2.  Some twenty-five symmetric products, which run on digits,
+// in place of a tridiagonal eigenproblem bound by FP64 latency.  The elements of X stay within [-1, 1],
+// so its digits need no row maxima and are cut by the pass that updates X.  False (X undefined) when the
+// spectrum has no gap there that 60 steps resolve, or is not finite; the caller then diagonalises.
+// Y: n x n of work.
+__device__ __noinline__ bool sc_purify(int n, int o, const double *F, double *X, double *Y, const ScDig &dg, ScShared &sm) {
+    const int lane = threadIdx.x & 31, gw = sm.rank * SC_W + (threadIdx.x >> 5), warps = SC_W * sm.csize;
+    double lo = 1e300, hi = -1e300;   // Gershgorin bounds
+    for (int i = gw; i < n; i += warps) {
+        double r = 0.0;
+        for (int j = lane; j < n; j += 32) r += j == i ? 0.0 : fabs(F[(long long)i * n + j]);
+        for (int off = 16; off; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+        const double d = F[(long long)i * n + i];
+        lo = fmin(lo, d - r);
+        hi = fmax(hi, d + r);
+    }
+    lo = -sc_max(-lo, sm);
+    hi = sc_max(hi, sm);
+    const double w = hi - lo;
+    if (!(w > 0.0) || !isfinite(w)) return false;   // the same in every thread of the cluster
+    const double s = 1.0 / w;
+    const bool dig = sc_digits(n, sm);
+    const int nt = (n + 15) / 16, g = lane >> 2, t = lane & 3;
+    // X = X_0 (mode 0), Y (1) or 2 X - Y (2), with its digits
+    auto update = [&](int mode) {
+        auto value = [&](int r, int k) {
+            const long long x = (long long)r * n + k;
+            const double v = mode == 0 ? s * ((r == k ? hi : 0.0) - F[x]) : mode == 1 ? Y[x] : 2.0 * X[x] - Y[x];
+            X[x] = v;
+            return v;
+        };
+        if (dig) {
+            for (int task = gw; task < nt * nt; task += warps) {
+                const int rt = task / nt, kt = task % nt;
+                unsigned long long y[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int r = rt * 16 + g + (q >> 2) * 8, k = kt * 16 + 2 * t + ((q >> 1) & 1) * 8 + (q & 1);
+                    y[q] = cd_fixed(r < n && k < n ? value(r, k) : 0.0, 0);
+                }
+                sc_store(dg.a + ((long long)task * 8) * 32 + lane, y);
+            }
+        } else {
+            SC_FOR(x, (long long)n * n) value((int)(x / n), (int)(x % n));
+        }
+        sc_bar(sm);
+    };
+    if (dig) SC_FOR(r, nt * 16) dg.ea[r] = 0;
+    update(0);
+    double t1 = 0.0;
+    SC_FOR(i, n) t1 += X[i * n + i];
+    t1 = sc_sum(t1, sm);
+    bool prev = false, last = false;
+    for (int it = 0; it < 60; ++it) {
+        double t2 = 0.0;   // Y = X^2 and its trace
+        if (dig) {
+            t2 = sc_digit_gemm(n, n, n, 1.0, dg.a, dg.ea, dg.a, dg.ea, 0.0, Y, n, true, sm);
+        } else {
+            sc_gemm<double, ScTile<double>::R>(n, n, n, 1.0, X, n, false, X, n, true, 0.0, Y, n, sm, true);
+            SC_FOR(i, n) t2 += Y[i * n + i];
+        }
+        t2 = sc_sum(t2, sm);
+        if (sm.csize == 1) __syncthreads();
+        if (!isfinite(t2)) return false;
+        // the last step is the other one: eigenvalues off by d from 0 and from 1 are then both off by d^2
+        const bool square = last ? !prev : fabs(t2 - o) <= fabs(2.0 * t1 - t2 - o);
+        const bool near = fabs(t1 - t2) < 1e-8;
+        update(square ? 1 : 2);
+        t1 = square ? t2 : 2.0 * t1 - t2;
+        if (last) return fabs(t1 - o) < 1e-7;
+        last = near;
+        prev = square;
+    }
+    return false;
+}
+
 struct ScState {
     int it;            // iterations done (both phases)
     bool converged;
@@ -1006,9 +1309,9 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
         sc_charges<T>(n, N, w.P, w.S, w.gam, p0, sm);
         sc_fock<T>(n, N, a.lc != 0, w, p0, sm);
         // F' = X F X, E' = F' P' - P' F'
-        gemm<T>(n, n, n, T(1), w.X, n, false, w.F, n, false, T(0), w.T1, n, sm);
-        gemm_sym<T>(n, n, T(1), w.T1, n, false, w.X, n, false, T(0), w.Fp, n, sm);
-        gemm<T>(n, n, n, T(1), w.Fp, n, false, w.Pp, n, false, T(0), w.T1, n, sm);
+        sc_prod(w.dg, n, n, n, T(1), OP_X, w.X, n, false, OP_ANY, w.F, n, false, T(0), w.T1, n, false, sm);
+        sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.T1, n, false, OP_X, w.X, n, false, T(0), w.Fp, n, true, sm);
+        sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.Fp, n, false, OP_ANY, w.Pp, n, false, T(0), w.T1, n, false, sm);
         const int cur = hist % SC_DIIS;
         T *Fc = w.Fh + cur * nn, *Ec = w.Eh + cur * nn;
         double emax = 0.0;
@@ -1069,14 +1372,24 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
             w.EA[t] = v;
         }
         sc_bar(sm);
-        if (!sc_eigh<T>(n, o, w.EA, w.Z, w.W, piv, sm)) {
+        if constexpr (sizeof(T) == 8) {
+            // P' = 2 X, P = X_orth P' X_orth with X_orth = S^-1/2
+            if (sm.csize > 1 && sc_purify(n, o, w.EA, w.Pp, w.T1, w.dg, sm)) {
+                SC_FOR(t, nn) w.Pp[t] *= T(2);
+                sc_bar(sm);
+                sc_prod(w.dg, n, n, n, T(1), OP_X, w.X, n, false, OP_ANY, w.Pp, n, false, T(0), w.T1, n, false, sm);
+                sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.T1, n, false, OP_X, w.X, n, false, T(0), w.P, n, true, sm);
+                continue;
+            }
+        }
+        if (!sc_eigh<T>(n, o, w.EA, w.Z, w.W, piv, w.dg, sm)) {
             st.finite = false;
             return;
         }
         // P' = 2 Z Z^T, C_o = X Z, P = 2 C_o C_o^T
-        gemm_sym<T>(n, o, T(2), w.Z, o, false, w.Z, o, true, T(0), w.Pp, n, sm);
-        gemm<T>(n, o, n, T(1), w.X, n, false, w.Z, o, false, T(0), w.T2, o, sm);
-        gemm_sym<T>(n, o, T(2), w.T2, o, false, w.T2, o, true, T(0), w.P, n, sm);
+        sc_prod(w.dg, n, n, o, T(2), OP_ANY, w.Z, o, false, OP_ANY, w.Z, o, true, T(0), w.Pp, n, true, sm);
+        sc_prod(w.dg, n, o, n, T(1), OP_X, w.X, n, false, OP_ANY, w.Z, o, false, T(0), w.T2, o, false, sm);
+        sc_prod(w.dg, n, n, o, T(2), OP_ANY, w.T2, o, false, OP_ANY, w.T2, o, true, T(0), w.P, n, true, sm);
     }
 }
 
@@ -1116,7 +1429,7 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
         // X = S^-1/2 and S^1/2 from the eigenpairs of S (scc_routine.rs:172-174)
         SC_FOR(t, nn) w.EA[t] = w.S[t];
         sc_bar(sm);
-        bool ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, sm);
+        bool ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, w.dg, sm);
         if (ok) {
             double bad = 0.0;
             for (int r = tid; r < n; r += SC_T) bad = fmax(bad, sm.w[r] > 0.0 ? 0.0 : 1.0);
@@ -1139,6 +1452,10 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
             sc_bar(sm);
             gemm_sym<double>(n, n, 1.0, w.T1, n, false, w.Z, n, true, 0.0, w.X, n, sm);
             gemm_sym<double>(n, n, 1.0, w.T2, n, false, w.Z, n, true, 0.0, w.Sh, n, sm);
+            if (sc_digits(n, sm)) {
+                sc_split(w.S, n, false, n, n, w.dg.S, w.dg.eS, sm);
+                sc_split(w.X, n, false, n, n, w.dg.X, w.dg.eX, sm);
+            }
             start_density();
         }
         int remaining = a.max_iter, hist = 0;
@@ -1199,7 +1516,7 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
             // orbitals of the last Fock matrix (scc_routine.rs:187-192)
             SC_FOR(t, nn) w.EA[t] = w.Fp[t];
             sc_bar(sm);
-            ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, sm);
+            ok = sc_eigh<double>(n, n, w.EA, w.Z, w.Fh, sl.piv, w.dg, sm);
         }
         if (ok) {
             double *C = a.orbs + sy.mat_off;
@@ -1336,9 +1653,9 @@ int Ctx::scc_batch(int n_sys, const tincr_scc_system *sys, const int *kinds, con
     // slots
     const long long nn_max = (long long)nmax * nmax, at2_max = (long long)Nmax * Nmax, npad = (nmax + 31) / 32 * 32;
     const long long slot_bytes =
-        (sc_slot_doubles(nn_max, at2_max, npad) * (long long)sizeof(double) + nn_max + 255) / 256 * 256;
+        (sc_slot_doubles(nn_max, at2_max, npad) * (long long)sizeof(double) + nn_max + 255) / 256 * 256 + sc_digit_bytes(npad);
     // CTAs per system
-    int csize = 1;
+    int csize = 2;
     while (csize < SC_CMAX && 2LL * csize * n_sys <= SC_FILL * n_sm) csize *= 2;
     const int n_slots = std::min(n_sys, SC_SLOTS_PER_SM * n_sm / csize);
     scc_ws.reserve((size_t)(slot_bytes * n_slots));
