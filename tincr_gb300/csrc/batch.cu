@@ -790,11 +790,11 @@ __device__ __forceinline__ void bt_block_sum(double (&v)[NV], double *red) {
     __syncthreads();
 }
 
-// sum over the CTA of eight values per thread; every thread receives the totals.  Within a warp the
-// eight sums are reduced by halving exchanges (lanes 0-15 keep values 0-3 and receive them from lanes
-// 16-31, and so on): 9 shuffle-adds instead of 40.  red: (BT_T / 32 + 1) * 8 doubles.
-__device__ __forceinline__ void bt_block_sum8(double (&v)[8], double *red) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// sums over a warp of eight values per thread into out[0 .. 7].  The eight sums are reduced by halving
+// exchanges (lanes 0-15 keep values 0-3 and receive them from lanes 16-31, and so on): 9 shuffle-adds
+// instead of 40.
+__device__ __forceinline__ void bt_warp_sum8(const double (&v)[8], double *out) {
+    const int lane = threadIdx.x & 31;
     const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
     double a[4], b[2], c;
 #pragma unroll
@@ -814,19 +814,7 @@ __device__ __forceinline__ void bt_block_sum8(double (&v)[8], double *red) {
     c += __shfl_xor_sync(0xffffffffu, c, 2);
     c += __shfl_xor_sync(0xffffffffu, c, 1);
     // lane L now holds the warp total of value (L >> 2) & 7
-    __syncthreads();
-    if ((lane & 3) == 0) red[warp * 8 + ((lane >> 2) & 7)] = c;
-    __syncthreads();
-    double *tot = red + (BT_T / 32) * 8;
-    if (threadIdx.x < 8) {
-        double s = 0.0;
-        for (int w = 0; w < BT_T / 32; ++w) s += red[w * 8 + threadIdx.x];
-        tot[threadIdx.x] = s;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = tot[q];
-    __syncthreads();
+    if ((lane & 3) == 0) out[(lane >> 2) & 7] = c;
 }
 
 // Number of eigenvalues of the symmetric tridiagonal (d, squared off-diagonal esq) below x: the
@@ -1310,20 +1298,28 @@ __global__ void __cluster_dims__(BT_CL, 1, 1) __launch_bounds__(BT_T)
             double *t = T + (long long)j * ov;
             const int mc = s_mcur;
             double *part = cbuf[ph];
+            // The warps' sums of all dots first, then one pass over the warps: two barriers for all the dots
+            // instead of four per eight of them.  They lie in Z, whose last readers (bt_ritz) are behind the
+            // barriers of the residual norms: 8 rows of mmax + 8, at most mmax^2 from mmax = 15 on.
+            // Eight stacked acenes FP64 (4 + 1 roots), device time of the batch: 10.35 -> 10.0 ms.
             for (int i0 = 0; i0 < mc; i0 += 8) {
                 double c8[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) c8[q] = 0.0;
+#pragma unroll 2
                 for (long long x = x0; x < ov; x += xs) {
                     const double tx = t[x];
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         if (i0 + q < mc) c8[q] += V[(long long)(i0 + q) * ov + x] * tx;
                 }
-                bt_block_sum8(c8, red);
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    if (tid == q) part[i0 + q] = c8[q];
+                bt_warp_sum8(c8, Z + (size_t)(tid >> 5) * (mmax + 8) + i0);
+            }
+            __syncthreads();
+            for (int i = tid; i < mc; i += BT_T) {
+                double s = 0.0;
+                for (int w = 0; w < BT_T / 32; ++w) s += Z[(size_t)w * (mmax + 8) + i];
+                part[i] = s;
             }
             bt_cluster_sum(cl, coop, part, mc, cdot);
             ph ^= 1;
