@@ -267,6 +267,9 @@ __global__ void row_sq_finish_kernel(int rows, int chunks, const double *__restr
 // the same fixed order and takes the same decision; when t'_j is accepted its dot with t_{j+1} joins
 // the next coefficients.  Normalisation is deferred: an accepted row is kept as t' with the factor
 // 1/|t'|, which the coefficients apply, and every accepted row is scaled in place at the end.
+// Bound by waits: three to four elements per thread and pass, a barrier per vector, the FP64 sums.  The
+// accepted rows are loaded eight at a time before the first is used, so that a thread waits for the L2
+// once per eight rows (ov = 131072, 51 launches of a 20-root solve: 11.1 -> 6.7 ms).
 // state[0]: m out; state[1]: 1 if a norm was not finite.  part: [2][gridDim.x][GS_SLOTS] doubles.
 constexpr int GS_MAX = 32, GS_SLOTS = GS_MAX + 2;
 __global__ void __launch_bounds__(256) seq_gs_kernel(int kadd, long long ov, int m0, int mmax, double *V, double *T,
@@ -293,12 +296,18 @@ __global__ void __launch_bounds__(256) seq_gs_kernel(int kadd, long long ov, int
             double v = t[x];
             const double tnx = tn ? tn[x] : 0.0;
 #pragma unroll
-            for (int i = 0; i < GS_MAX; ++i)
-                if (i < acc) {
-                    const double q = V[(long long)(m0 + i) * ov + x];
-                    if (i < ncoef) v -= c[i] * q;
-                    d[i] += q * tnx;
-                }
+            for (int i0 = 0; i0 < GS_MAX; i0 += 8) {
+                if (i0 >= acc) break;
+                double q[8];   // eight rows in flight: one after the other each waits for the L2
+#pragma unroll
+                for (int r = 0; r < 8; ++r) q[r] = i0 + r < acc ? V[(long long)(m0 + i0 + r) * ov + x] : 0.0;
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    if (i0 + r < acc) {
+                        if (i0 + r < ncoef) v -= c[i0 + r] * q[r];
+                        d[i0 + r] += q[r] * tnx;
+                    }
+            }
             dst[x] = v;
             sq += v * v;
             d[GS_MAX] += v * tnx;
@@ -1012,7 +1021,8 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                 if (kadd <= 32 && coop_grid > 0) {
                     int slot = prof_begin(TINCR_KF_SUBSPACE);
                     // no more CTAs than blocks of 256 elements: each barrier and each sum over the CTAs is
-                    // shorter, and empty CTAs only add zeros (C20H22, 10 corrections: 142 -> 132 us)
+                    // shorter, and empty CTAs only add zeros (C20H22, 10 corrections: 142 -> 132 us before the rows
+                    // were loaded in groups)
                     const int gs_grid = (int)std::min<long long>(coop_grid, (ov + 255) / 256);
                     gs_part.reserve((size_t)2 * coop_grid * GS_SLOTS);
                     gs_state.reserve(2);
