@@ -269,9 +269,36 @@ __global__ void row_sq_finish_kernel(int rows, int chunks, const double *__restr
 // 1/|t'|, which the coefficients apply, and every accepted row is scaled in place at the end.
 // Bound by waits: three to four elements per thread and pass, a barrier per vector, the FP64 sums.  The
 // accepted rows are loaded eight at a time before the first is used, so that a thread waits for the L2
-// once per eight rows (ov = 131072, 51 launches of a 20-root solve: 11.1 -> 6.7 ms).
+// once per eight rows (ov = 131072, 51 launches of a 20-root solve: 11.1 -> 6.7 ms), and only the slots in use are summed over the warps.
 // state[0]: m out; state[1]: 1 if a norm was not finite.  part: [2][gridDim.x][GS_SLOTS] doubles.
 constexpr int GS_MAX = 32, GS_SLOTS = GS_MAX + 2;
+
+// Sums over a warp of d[0 .. NS) (NS = 8, 16 or 32) into out[0 .. NS): at each lane bit from 16 down a lane
+// keeps half of its values and receives that half from its partner; once one value is left the rest is
+// a butterfly.  9, 16 or 31 shuffle-adds: GB300's FP64 unit takes ~64 cycles per warp instruction (a whole
+// solve of C20H22, 10 roots FP64, with 32 slots always: 2.29 ms, by the slots in use: 2.20 ms).
+template <int NS>
+__device__ __forceinline__ void gs_warp_sums(const double (&d)[GS_MAX + 1], double *out) {
+    const int lane = threadIdx.x & 31;
+    double v[NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) v[q] = d[q];
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+        const int off = 16 >> b, half = (NS >> b) / 2;
+        if (half) {
+            const bool h = lane & off;
+#pragma unroll
+            for (int q = 0; q < half; ++q)
+                v[q] = (h ? v[q + half] : v[q]) + __shfl_xor_sync(0xffffffffu, h ? v[q] : v[q + half], off);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+        }
+    }
+    // lane L holds slot L / (32 / NS)
+    if (lane % (32 / NS) == 0) out[lane / (32 / NS)] = v[0];
+}
+
 __global__ void __launch_bounds__(256) seq_gs_kernel(int kadd, long long ov, int m0, int mmax, double *V, double *T,
                                                      double *part, int *state) {
     cg::grid_group grid = cg::this_grid();
@@ -313,42 +340,17 @@ __global__ void __launch_bounds__(256) seq_gs_kernel(int kadd, long long ov, int
             d[GS_MAX] += v * tnx;
         }
         // block partials: slots 0 .. acc-1 (dots with q_i), GS_MAX (dot with t'_j), GS_MAX + 1 (|t'_j|^2).
-        // The 32 dot slots are reduced over the warp by halving exchanges (lane L ends with slot L:
-        // 31 shuffle-adds instead of 160; GB300's FP64 unit takes ~64 cycles per warp instruction).
+        // The dot slots in use, rounded up to 8, 16 or 32, are reduced over the warp by halving exchanges; the
+        // tree over the lanes is the same for each count, and so are the bits.
         double *pb = part + ((long long)(j & 1) * gridDim.x + blockIdx.x) * GS_SLOTS;
+        if (acc <= 8) gs_warp_sums<8>(d, red[warp]);
+        else if (acc <= 16) gs_warp_sums<16>(d, red[warp]);
+        else gs_warp_sums<32>(d, red[warp]);
         {
-            double a16[16], a8[8], a4[4], a2[2];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const bool h = lane & 16;
-                a16[q] = (h ? d[q + 16] : d[q]) + __shfl_xor_sync(0xffffffffu, h ? d[q] : d[q + 16], 16);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const bool h = lane & 8;
-                a8[q] = (h ? a16[q + 8] : a16[q]) + __shfl_xor_sync(0xffffffffu, h ? a16[q] : a16[q + 8], 8);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const bool h = lane & 4;
-                a4[q] = (h ? a8[q + 4] : a8[q]) + __shfl_xor_sync(0xffffffffu, h ? a8[q] : a8[q + 4], 4);
-            }
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const bool h = lane & 2;
-                a2[q] = (h ? a4[q + 2] : a4[q]) + __shfl_xor_sync(0xffffffffu, h ? a4[q] : a4[q + 2], 2);
-            }
-            const bool h = lane & 1;
-            red[warp][lane] = (h ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, h ? a2[0] : a2[1], 1);
-            double vc = d[GS_MAX], vs = sq;
-            for (int off = 16; off; off >>= 1) {
-                vc += __shfl_xor_sync(0xffffffffu, vc, off);
-                vs += __shfl_xor_sync(0xffffffffu, vs, off);
-            }
-            if (lane == 0) {
-                red[warp][GS_MAX] = vc;
-                red[warp][GS_MAX + 1] = vs;
-            }
+            const bool h = lane & 16;
+            double v = (h ? sq : d[GS_MAX]) + __shfl_xor_sync(0xffffffffu, h ? d[GS_MAX] : sq, 16);
+            for (int off = 8; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if ((lane & 15) == 0) red[warp][GS_MAX + (lane >> 4)] = v;
         }
         __syncthreads();
         if (threadIdx.x < GS_SLOTS && (threadIdx.x < acc || threadIdx.x >= GS_MAX)) {
