@@ -5,8 +5,10 @@
 // GB300's FP64 pipe (~2 DFMA per SM clock), pays for the padding in time; these kernels keep the
 // short dimension exact.
 //
-// skinny_dots:  C[i][j] += sum_x A[i][x] B[j][x]   (i < M, j < NB <= 32), L split across CTAs,
-//               32 x NB output block per CTA staged through shared memory, FP64 atomics into C.
+// skinny_dots:  C[i][j] = sum_x A[i][x] B[j][x]   (i < M, j < NB <= 32), L split across CTAs,
+//               32 x NB output block per CTA staged through shared memory; the CTAs' sums are added in a
+//               fixed order by skinny_sum_kernel, so equal inputs give equal bits (FP64 atomics into C
+//               did not from three CTAs on).
 // skinny_comb:  Out[r][x] = epi(r, x, sum_i Y[r][i] V[i][x])   (r < R <= 32), one column per
 //               thread, Y staged in shared memory by 64-wide i chunks, coalesced reads of V rows.
 // Both are bound by the FP64 pipe of the SMs that have a CTA, so short vectors are cut finer: dots down
@@ -21,11 +23,12 @@ namespace tincr {
 constexpr int SK_ROWS = 32, SK_COLS = 64, SK_T = 256;
 constexpr int SK_FULL = 152;   // SMs of a GB300
 
-// C[M x nb] += A[M x L] . B[nb x L]^T ; rows of B at or beyond nb are read as zero.
+// out[x chunk][M x nb] = A[M x L] . B[nb x L]^T over the chunk, leading dimension ld; rows of B at or
+// beyond nb are read as zero.
 template <int NB>
 __global__ void __launch_bounds__(SK_T)
 skinny_dots_guard_kernel(int M, int nb, int L, int l_chunk, const double *__restrict__ A, long long lda,
-                         const double *__restrict__ B, long long ldb, double *C, int ldc) {
+                         const double *__restrict__ B, long long ldb, double *out, int ld) {
     __shared__ double As[SK_ROWS][SK_COLS + 1];
     __shared__ double Bs[NB][SK_COLS + 1];
     const int i0 = blockIdx.y * SK_ROWS;
@@ -61,8 +64,30 @@ skinny_dots_guard_kernel(int M, int nb, int L, int l_chunk, const double *__rest
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             int j = tj + 8 * k;
-            if (j < nb) atomicAdd(C + (long long)gi * ldc + j, acc[k]);
+            if (j < nb) out[((long long)blockIdx.x * M + gi) * ld + j] = acc[k];
         }
+}
+
+constexpr int SK_LANES = SK_T / 32;   // parts of a sum over the chunks
+
+// C[i][j] = sum over the chunks c of part[c][i][j]: warp w adds the chunks w, w + 8, ... of 32 outputs, the
+// first warp the eight sums in order.
+static __global__ void __launch_bounds__(SK_T)
+skinny_sum_kernel(int M, int nb, int chunks, const double *__restrict__ part, double *C, int ldc) {
+    __shared__ double red[SK_LANES][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = (long long)M * nb, t = blockIdx.x * 32LL + lane;
+    double s = 0.0;
+    if (t < total)
+#pragma unroll 4
+        for (int c = w; c < chunks; c += SK_LANES) s += part[c * total + t];
+    red[w][lane] = s;
+    __syncthreads();
+    if (w > 0 || t >= total) return;
+    s = red[0][lane];
+#pragma unroll
+    for (int q = 1; q < SK_LANES; ++q) s += red[q][lane];
+    C[t / nb * ldc + t % nb] = s;
 }
 
 // Out[r][x] = epi(r, x, sum_{i < m} Y(r, i) V[i][x]),  r < R (template, <= 32),
@@ -125,8 +150,9 @@ struct CombResidual {           // Rk[r][x] = acc - u[r] R[r][x]
 
 // launchers ----------------------------------------------------------------------------------
 
+// part: workspace for the sums of the chunks
 inline void skinny_dots(cudaStream_t st, int n_sm, int M, int nb, long long L, const double *A, long long lda,
-                        const double *B, long long ldb, double *C, int ldc) {
+                        const double *B, long long ldb, double *C, int ldc, DevBuf<double> &part) {
     if (M <= 0 || nb <= 0 || L <= 0) return;
     int my = ceil_div(M, SK_ROWS);
     long long want = 2LL * n_sm;                       // CTAs in flight
@@ -134,14 +160,23 @@ inline void skinny_dots(cudaStream_t st, int n_sm, int M, int nb, long long L, c
     int l_chunk = (int)(((L + chunks - 1) / chunks + SK_COLS - 1) / SK_COLS * SK_COLS);
     int gx = (int)((L + l_chunk - 1) / l_chunk);
     dim3 grid(gx, my);
+    // gx M <= 32 (want + my): one size for every call up to 64 row blocks
+    if (gx > 1) part.reserve((size_t)(want + std::max(my, 64)) * SK_ROWS * 32);
+    double *out = gx > 1 ? part.p : C;
+    const int ld = gx > 1 ? nb : ldc;
     // the FP64 pipe is the bound: the instantiation closest above nb wastes the fewest FMAs
-    if (nb <= 8) skinny_dots_guard_kernel<8><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, C, ldc);
-    else if (nb <= 16) skinny_dots_guard_kernel<16><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, C, ldc);
-    else if (nb <= 24) skinny_dots_guard_kernel<24><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, C, ldc);
-    else if (nb <= 32) skinny_dots_guard_kernel<32><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, C, ldc);
+    if (nb <= 8) skinny_dots_guard_kernel<8><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, out, ld);
+    else if (nb <= 16) skinny_dots_guard_kernel<16><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, out, ld);
+    else if (nb <= 24) skinny_dots_guard_kernel<24><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, out, ld);
+    else if (nb <= 32) skinny_dots_guard_kernel<32><<<grid, SK_T, 0, st>>>(M, nb, (int)L, l_chunk, A, lda, B, ldb, out, ld);
     else fail(TINCR_BAD_ARG, "skinny_dots: more than 32 short rows");
     count_launch(st, "skinny_dots");
     check_launch("skinny_dots");
+    if (gx > 1) {
+        skinny_sum_kernel<<<(unsigned)(((long long)M * nb + 31) / 32), SK_T, 0, st>>>(M, nb, gx, part.p, C, ldc);
+        count_launch(st, "skinny_sum");
+        check_launch("skinny_sum");
+    }
 }
 
 template <class Epi>

@@ -909,13 +909,13 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
         if (knew > 0 && dg) {
             dg_project(m, mold, knew, dAp.p, mmax);
         } else if (knew > 0) {
-            TINCR_CUDA(cudaMemset2DAsync(dAp.p + mold, (size_t)mmax * sizeof(double), 0, (size_t)knew * sizeof(double),
-                                         m, stream));
             if (knew <= 32) {
                 int slot = prof_begin(TINCR_KF_SUBSPACE);
-                skinny_dots(stream, n_sm, m, knew, ov, dV.p, ov, dAV.p + (long long)mold * ov, ov, dAp.p + mold, mmax);
+                skinny_dots(stream, n_sm, m, knew, ov, dV.p, ov, dAV.p + (long long)mold * ov, ov, dAp.p + mold, mmax, sk_part);
                 prof_end(slot, 2.0 * m * (double)knew * ov, 8.0 * (double)(m + knew) * ov);
             } else {
+                TINCR_CUDA(cudaMemset2DAsync(dAp.p + mold, (size_t)mmax * sizeof(double), 0,
+                                             (size_t)knew * sizeof(double), m, stream));
                 int sk = pick_splitk(m, knew, (int)ov, 1, n_sm);
                 pgemm<false, true>(*this, TINCR_KF_SUBSPACE, m, knew, (int)ov, dV.p, (int)ov, 0,
                                    dAV.p + (long long)mold * ov, (int)ov, 0, 1, EpiAtomicAdd{dAp.p + mold, 0, mmax, 1.0}, sk);
@@ -1005,10 +1005,9 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                 if (dg) {
                     dg_ortho(kadd, m, dT.p, dc.p);
                 } else if (kadd <= 32) {
-                    TINCR_CUDA(cudaMemsetAsync(dc.p, 0, (size_t)kadd * m * sizeof(double), stream));
                     // c = V T^T  [m x kadd];  T -= c^T V
                     int slot = prof_begin(TINCR_KF_SUBSPACE);
-                    skinny_dots(stream, n_sm, m, kadd, ov, dV.p, ov, dT.p, ov, dc.p, kadd);
+                    skinny_dots(stream, n_sm, m, kadd, ov, dV.p, ov, dT.p, ov, dc.p, kadd, sk_part);
                     skinny_comb(stream, kadd, m, ov, dc.p, 1, kadd, dV.p, ov, CombStore{dT.p, ov, -1.0, 1.0});
                     prof_end(slot, 4.0 * kadd * (double)m * ov, 8.0 * (2.0 * m + 3.0 * kadd) * ov);
                 } else {
@@ -1050,10 +1049,9 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                         double *t = dT.p + (long long)j * ov;
                         int acc = m - m0;
                         if (acc > 0) {
-                            TINCR_CUDA(cudaMemsetAsync(dc.p, 0, acc * sizeof(double), stream));
                             // c = Q t  [acc x 1] over the vectors accepted in this step;  t -= c^T Q
                             int slot = prof_begin(TINCR_KF_SUBSPACE);
-                            skinny_dots(stream, n_sm, acc, 1, ov, dV.p + (long long)m0 * ov, ov, t, ov, dc.p, 1);
+                            skinny_dots(stream, n_sm, acc, 1, ov, dV.p + (long long)m0 * ov, ov, t, ov, dc.p, 1, sk_part);
                             skinny_comb(stream, 1, acc, ov, dc.p, acc, 1, dV.p + (long long)m0 * ov, ov,
                                         CombStore{t, ov, -1.0, 1.0});
                             prof_end(slot, 4.0 * acc * (double)ov, 8.0 * (acc + 2.0) * ov);

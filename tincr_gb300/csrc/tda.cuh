@@ -165,7 +165,7 @@ struct Ctx {
     explicit Ctx(int dev);
     ~Ctx();
     void sync();
-    DevBuf<double> norm_partial, gs_part;
+    DevBuf<double> norm_partial, gs_part, sk_part;
     DevBuf<int> gs_state;
     int coop_grid = 0;                    // CTAs of the cooperative Gram-Schmidt launch
     void row_norms(int rows, long long len, const double *A, long long lda, double *out);
