@@ -10,7 +10,7 @@
 // Fock matrix (up to 8 iterates).  tincr mixes Mulliken charges with Broyden's method and stops at an
 // rms charge change of 1e-5: the same stationary density, reached here to a tighter test.
 //
-// Layout.  A persistent grid of clusters (two CTAs per SM) takes systems from a counter, largest first.
+// Layout.  A persistent grid of clusters of 1 to 16 CTAs (two CTAs per SM) takes systems from a counter, largest first.
 // A cluster keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and
 // runs every step itself; its CTAs share out the tiles, rows, roots and elements of a step and meet at
 // the cluster barrier, small vectors and sums going straight into each other's shared memory:
@@ -24,8 +24,7 @@
 //    pivoting), Loewdin's orthogonalisation to first order (Gram-Schmidt inside clusters of close roots
 //    where that does not do), and the back-transformation by the stored reflections;
 //  * the Fock build, Mulliken charges, DIIS and the energy as element loops and reductions.
-// CTAs per system: the largest power of two from 2 to 16 that keeps the batch within SC_FILL CTAs per SM.
-// Kernel time (ms, LC, to 1e-10) with one CTA per system, FP64 tiles and the eigensolver in every
+// CTAs per system: sc_ctas_per_system.  Kernel time (ms, LC, to 1e-10) with one CTA per system, FP64 tiles and the eigensolver in every
 // iteration / with clusters / with digit products and purification too:
 //     one decacene (192 orbitals)  705 / 123 / 44       128 acene dimers (up to 186)  750 / 417 / 176
 //     16 acene dimers              690 / 160 / 54       64 acenes (up to 102)         145 /  74 /  37
@@ -69,7 +68,8 @@ constexpr int SC_SLOTS_PER_SM = 2;
 constexpr int SC_KS = 32;              // k depth of a GEMM slice
 constexpr int SC_DIGITS = 20000;       // n^3 per CTA from which the iterations' FP64 products run on digits
 constexpr int SC_CMAX = 16;            // CTAs per cluster
-constexpr int SC_FILL = 4;             // CTAs per SM that a batch is spread over (twice those that run at once)
+constexpr int SC_FILL = 4;             // CTAs per SM that a batch of large systems is spread over (twice those that run at once)
+constexpr double SC_SMALL = 96.0;      // orbitals below which systems count as small (sc_ctas_per_system)
 
 struct ScArgs {
     int n_sys;
@@ -1374,7 +1374,7 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
         sc_bar(sm);
         if constexpr (sizeof(T) == 8) {
             // P' = 2 X, P = X_orth P' X_orth with X_orth = S^-1/2
-            if (sm.csize > 1 && sc_purify(n, o, w.EA, w.Pp, w.T1, w.dg, sm)) {
+            if (sc_purify(n, o, w.EA, w.Pp, w.T1, w.dg, sm)) {
                 SC_FOR(t, nn) w.Pp[t] *= T(2);
                 sc_bar(sm);
                 sc_prod(w.dg, n, n, n, T(1), OP_X, w.X, n, false, OP_ANY, w.Pp, n, false, T(0), w.T1, n, false, sm);
@@ -1566,6 +1566,34 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
     }
 }
 
+// CTAs per system, one for the whole batch: the largest power of two that keeps it within `fill` CTAs per SM.
+// What the size of its systems allows is measured by their mean weighted with the cube, the work of an
+// iteration (a few large systems decide, a few large ones among thousands of small ones do not).  Below 16
+// orbitals a second CTA only adds barriers; below SC_SMALL the systems of a batch converge alike, so more
+// than what runs at once is a second wave, while the larger ones (dimers) differ by hundreds of iterations
+// and the last ones are worth the CTAs.  Clusters of 16 fit on a GPC a few at a time, so small systems take
+// them up to four.  Kernel time (ms, LC, to 1e-10) with one CTA and the eigensolver in every iteration / two
+// CTAs and more, SC_FILL CTAs per SM for all / this rule:
+//     304 systems of 6 orbitals  1.74 / 3.89 / 1.51     304 of 30 orbitals  11.5 / 16.5 /  8.1
+//      64 of 6                   1.60 / 3.73 / 1.26     152 of 30           10.3 / 15.5 /  6.3
+//     304 of 12                  2.79 / 4.75 / 1.96     152 of 48           23.0 / 32.3 / 14.3
+//     304 of 24                  6.83 / 8.55 / 5.03     152 of 66           56.9 / 48.5 / 28.6
+int sc_ctas_per_system(int n_sys, const tincr_scc_system *sys, int n_sm) {
+    double w3 = 0.0, w4 = 0.0;
+    for (int i = 0; i < n_sys; ++i) {
+        const double n = sys[i].n_orb;
+        w3 += n * n * n;
+        w4 += n * n * n * n;
+    }
+    const double size = w4 / w3;
+    const bool small = size < SC_SMALL;
+    const int fill = size < 32.0 ? 1 : small ? 2 : SC_FILL;
+    const int most = size < 16.0 ? 1 : size < 32.0 ? 4 : small && n_sys > 4 ? 8 : SC_CMAX;
+    int csize = small ? 1 : 2;
+    while (csize < most && 2LL * csize * n_sys <= (long long)fill * n_sm) csize *= 2;
+    return csize;
+}
+
 }  // namespace
 
 int Ctx::scc_batch(int n_sys, const tincr_scc_system *sys, const int *kinds, const double *xyz,
@@ -1654,9 +1682,7 @@ int Ctx::scc_batch(int n_sys, const tincr_scc_system *sys, const int *kinds, con
     const long long nn_max = (long long)nmax * nmax, at2_max = (long long)Nmax * Nmax, npad = (nmax + 31) / 32 * 32;
     const long long slot_bytes =
         (sc_slot_doubles(nn_max, at2_max, npad) * (long long)sizeof(double) + nn_max + 255) / 256 * 256 + sc_digit_bytes(npad);
-    // CTAs per system
-    int csize = 2;
-    while (csize < SC_CMAX && 2LL * csize * n_sys <= SC_FILL * n_sm) csize *= 2;
+    const int csize = sc_ctas_per_system(n_sys, sys, n_sm);
     const int n_slots = std::min(n_sys, SC_SLOTS_PER_SM * n_sm / csize);
     scc_ws.reserve((size_t)(slot_bytes * n_slots));
     ScArgs a{};
