@@ -1,0 +1,68 @@
+"""The batched SCC where occupied and virtual level coincide: the purification finds no gap and the iteration
+falls back on the eigenpairs, at every number of CTAs per system; the result is still a closed-shell density of
+the lowest orbitals.  With S and H0 given and no charge interaction the Fock matrix is H0 itself, so the
+orbital energies and the energy are known."""
+
+import numpy as np
+import pytest
+
+from tincr_gb300 import _lib
+from tincr_gb300 import geometry as G
+from tincr_gb300 import groundstate as gs
+from tincr_gb300 import scc as gscc
+
+
+def _degenerate(rings, lc, gap, seed):
+    """A System with given matrices whose frontier levels are `gap` apart, and its orbital energies."""
+    z, x = G.acene(rings)
+    sy = gs.build_system(z, G.to_bohr(x), lc=lc)
+    n, o = sy.n_orbs, sy.n_elec // 2
+    rng = np.random.default_rng(seed)
+    a = rng.normal(size=(n, n))
+    s = np.eye(n) + 0.02 * (a + a.T) / np.sqrt(n)
+    w, v = np.linalg.eigh(s)
+    assert w.min() > 0.5
+    sh = (v * np.sqrt(w)) @ v.T
+    eps = np.sort(rng.uniform(-1.0, 1.0, size=n))
+    eps[o] = eps[o - 1] + gap
+    eps[o + 1:] += max(0.0, eps[o] - eps[o + 1]) + 0.05
+    q, _ = np.linalg.qr(rng.normal(size=(n, n)))
+    h0 = sh @ ((q * eps) @ q.T) @ sh
+    na = sy.n_atoms
+    return sy, dict(s=(s + s.T) / 2, h0=(h0 + h0.T) / 2, gamma=np.zeros((na, na)), gamma_lr=np.zeros((na, na))), eps
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lc", [True, False])
+@pytest.mark.parametrize("rings,count", [(1, 1), (4, 1), (4, 6), (4, 30), (4, 70), (4, 160), (6, 1), (6, 160)])
+@pytest.mark.parametrize("gap", [0.0, 1e-9])
+def test_scc_of_degenerate_frontier_levels(gpu_ctx, rings, count, lc, gap):
+    sy, given, eps = _degenerate(rings, lc, gap, 100 * rings + count)
+    o, s = sy.n_elec // 2, given["s"]
+    got, rc = gscc.scc_batch(gpu_ctx, [sy] * count, tol=1e-10, given=[given] * count, max_iter=30)
+    assert rc == _lib.OK
+    energy = 2.0 * eps[:o].sum() + gs.repulsive_energy(sy)
+    for g in got:
+        assert g.converged
+        # sums of n terms of order one, errors of a few n eps
+        assert abs(np.sum(g.p * s) - 2.0 * o) < 1e-11
+        assert np.max(np.abs(g.p @ s @ g.p - 2.0 * g.p)) < 1e-11
+        assert np.max(np.abs(g.orbs.T @ s @ g.orbs - np.eye(sy.n_orbs))) < 1e-11
+        assert np.max(np.abs(g.orbe - eps)) < 1e-11
+        assert abs(np.sum(g.p * given["h0"]) - 2.0 * eps[:o].sum()) < 1e-10
+        assert abs(g.energy - energy) < 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lc", [True, False])
+def test_scc_of_two_separate_atoms(gpu_ctx, lc):
+    """Two H atoms out of range of each other: one level of two is filled whichever the eigensolver takes, so
+    the energy and the number of electrons are the host's."""
+    sy = gs.build_system(np.array([1, 1]), np.array([[0.0, 0, 0], [15.0, 0, 0]]), lc=lc)
+    h = gs.run_scc(sy, tol=1e-10, max_iter=30)
+    got, rc = gscc.scc_batch(gpu_ctx, [sy], tol=1e-10, max_iter=30)
+    # with LC the mixing of the two levels decays slowly (1e-8 after 30 iterations), its energy with the square
+    assert rc == _lib.OK or (lc and rc == _lib.NOT_CONVERGED)
+    assert abs(got[0].energy - h.energy) < 1e-12
+    assert abs(np.sum(got[0].p * got[0].s) - 2.0) < 1e-13
+    assert np.max(np.abs(got[0].orbe - h.orbe)) < 1e-12
