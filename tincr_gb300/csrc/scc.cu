@@ -1222,7 +1222,7 @@ __device__ __noinline__ bool sc_purify(int n, int o, const double *F, double *X,
         for (int off = 16; off; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
         const double d = F[(long long)i * n + i];
         lo = fmin(lo, d - r);
-        hi = fmax(hi, d + r);
+        hi = isfinite(d) && isfinite(r) ? fmax(hi, d + r) : HUGE_VAL;   // fmin and fmax drop a NaN
     }
     lo = -sc_max(-lo, sm);
     hi = sc_max(hi, sm);
