@@ -1166,7 +1166,10 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
         }
     }
     for (auto &v : tab) std::vector<int>().swap(v);
-    // device data of the exchange pass, which runs on while the host packs the next stage's inputs
+    // host lists and device data of the exchange pass, which runs on while the host packs the next stage's
+    // inputs; the lists come first, so that an error on the way frees them after the device (cudaFree waits)
+    std::vector<int> el_begin;
+    std::vector<int4> vt;
     DevBuf<double> d1;
     DevBuf<float> f32;
     DevBuf<ExMono> dm;
@@ -1175,8 +1178,6 @@ int Ctx::exciton_states(int n_mono, const tincr_exciton_monomer *mono, int n_pai
     DevBuf<ExEl> del;
     DevBuf<int> deb;
     DevBuf<int4> dvt;
-    std::vector<int> el_begin;
-    std::vector<int4> vt;
     auto run_exchange = [&](auto zero) {
         using T = decltype(zero);
         if (elv.empty()) return;
