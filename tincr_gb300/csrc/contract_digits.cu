@@ -284,7 +284,7 @@ DgOperand Ctx::cd_swpT(int blk) const {
 bool Ctx::digits_pay(int k, int R, int S, int P, int Q, bool exch) const {
     const double n = n_orb, nr = bsz(R), ns = bsz(S), np = bsz(P), nq = bsz(Q);
     const double mac = 2.0 * n * nr * ns + 2.0 * n * np * nq + (exch ? 4.0 * n * n * (ns + nq) : 0.0);
-    return use_digits && k * mac > CD_MIN_MAC;
+    return contract_digits && k * mac > CD_MIN_MAC;
 }
 
 void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q, double ax, double ac, double *out,

@@ -502,6 +502,9 @@ Ctx::Ctx(int dev) : device(dev) {
     // subspace products of the mixed Davidson: digit GEMMs on the tensor cores (default) or FP64
     const char *sg = std::getenv("TINCR_GB300_SUBSPACE_GEMM");
     if (sg && std::string(sg) == "fp64") use_digits = false;
+    // FP64 contraction of large work: digit GEMMs on the tensor cores (default) or FP64 tiles
+    const char *co = std::getenv("TINCR_GB300_CONTRACTION");
+    if (co && std::string(co) == "fp64") contract_digits = false;
 }
 
 Ctx::~Ctx() {

@@ -144,6 +144,7 @@ struct Ctx {
     int dg_check();
     // digit GEMMs of the FP64 contraction (contract_digits.cu): the system's orbital blocks, and the
     // workspace of a chunk of vectors
+    bool contract_digits = true;          // digit GEMMs where they pay, or FP64 tiles for all work
     bool cd_ready = false;
     DevBuf<__nv_bfloat16> cd_blk[2], cd_pl;
     DevBuf<int> cd_eblk[2], cd_int;
