@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) cd_max_kernel(CdSrc s, int rows_pad, unsi
     cd_load(s, blockIdx.z, blockIdx.y * 32, blockIdx.x * 64, x, st);
     unsigned m = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = max(m, cd_hi(x[j]));
+    for (int j = 0; j < 8; ++j) m = max(m, cd_hi_any(x[j]));
     for (int o = 4; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     const int r = blockIdx.y * 32 + (threadIdx.x >> 3);
     if ((threadIdx.x & 7) == 0 && m) atomicMax(mx + (long long)blockIdx.z * rows_pad + r, m);
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) cd_split_kernel(CdSrc s, int rows_pad, co
     if (blockIdx.x == 0 && (threadIdx.x & 7) == 0) E[row] = e;
     unsigned long long y[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) y[j] = cd_fixed(e == CD_POISON ? 0.0 : x[j], e);
+    for (int j = 0; j < 8; ++j) y[j] = cd_fixed<true>(e == CD_POISON ? 0.0 : x[j], e);
 #pragma unroll
     for (int p = 0; p < DG_PLANES; ++p) {
         unsigned w[4];
@@ -99,15 +99,29 @@ __global__ void __launch_bounds__(256) cd_split_kernel(CdSrc s, int rows_pad, co
     }
 }
 
+// sum over k of A(row, k) B(col, k) in FP64, k ascending: the results of a row without digits, which holds an
+// overflow of an earlier product
+__device__ __noinline__ double cd_direct(const CdSrc &A, const CdSrc &B, int b, int row, int col) {
+    const double *p = A.p + (long long)b * A.sb + (long long)row * A.rs;
+    const double *q = B.p + (long long)b * B.sb + (long long)col * B.rs;
+    double v = 0.0;
+    for (int k = 0; k < A.K; ++k) v = fma(p[(long long)k * A.ks], q[(long long)k * B.ks], v);
+    return v;
+}
+
 // Values of one thread's 16 results: A row `row` (bound Ea), B rows col0 .. col0 + 15 (bounds Eb)
 struct CdScale {
     const int *Ea, *Eb;   // per product: ea_b, eb_b entries further (0: shared)
     int ea_b, eb_b;
+    CdSrc A, B;           // what the digits were cut from
     __device__ __forceinline__ int row(int b, int r) const { return Ea[(long long)b * ea_b + r]; }
-    __device__ __forceinline__ double value(int b, int ea, int col, long long H, long long L) const {
+    __device__ __forceinline__ double value(int b, int row, int ea, int col, long long H, long long L) const {
         const int eb = Eb[(long long)b * eb_b + col];
-        if (ea == CD_POISON || eb == CD_POISON) return __longlong_as_double(0x7ff8000000000000ll);
-        return cd_value(H, L, ea + eb - 68);
+        const int e = ea + eb - 68;   // beyond every sum of two bounds where one row has no digits
+        return __longlong_as_double((long long)cd_value_bits(H, L, e, [&](unsigned long long m, int ex, unsigned long long s) {
+            if (e > CD_POISON / 2) return (unsigned long long)__double_as_longlong(cd_direct(A, B, b, row, col));
+            return cd_extreme(m, ex, s);
+        }));
     }
 };
 
@@ -129,10 +143,10 @@ struct CdEpiStore {
             if (col >= N) break;   // uniform over the warp
             double v = 0.0;
             if (row < M) {
-                v = sc.value(b, ea, col, H[j], L[j]);
+                v = sc.value(b, row, ea, col, H[j], L[j]);
                 C[(long long)b * sC + (long long)col * ld + row] = v;
             }
-            const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi(v));
+            const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi_any(v));
             if ((threadIdx.x & 31) == 0 && m) atomicMax(mx + (long long)b * mx_b + col, m);
         }
     }
@@ -160,13 +174,13 @@ struct CdEpiF {
             if (r >= n2) break;
             double f = 0.0;
             if (row < n2) {
-                const double v = sc.value(b, ea, r, H[j], L[j]);
+                const double v = sc.value(b, row, ea, r, H[j], L[j]);
                 const int rr = r < n ? r : r - n;
                 if (rr == cc && (r < n) != (row < n)) (r < n ? d3 : d2)[(long long)b * n + rr] = v;
                 f = ax * G[(long long)rr * n + cc] * v;
                 F[(long long)b * sF + (long long)r * ld + row] = f;
             }
-            const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi(f));
+            const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi_any(f));
             if ((threadIdx.x & 31) == 0 && m) atomicMax(mx + (long long)b * mx_b + r, m);
         }
     }
@@ -189,7 +203,7 @@ struct CdEpiOut {
         for (int j = 0; j < 16; ++j) {
             const int col = col0 + j;
             if (col >= N) break;
-            const double v = sc.value(b, ea, col, H[j], L[j]);
+            const double v = sc.value(b, row, ea, col, H[j], L[j]);
             const long long k = (long long)col * M + row;
             double *p = out + b * ov + k;
             if (X) *p = v + omega[k] * X[b * ov + k];
@@ -208,7 +222,7 @@ __global__ void __launch_bounds__(256) cd_scale_rows_kernel(int n, int nq, const
         v = z[(long long)b * n + (r < n ? r : r - n)] * Rv[(long long)r * nq + q];
         GT[((long long)b * nq + q) * ld + r] = v;
     }
-    const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi(v));
+    const unsigned m = __reduce_max_sync(0xffffffffu, cd_hi_any(v));
     if ((threadIdx.x & 31) == 0 && m) atomicMax(mx + (long long)b * mx_b + q, m);
 }
 
@@ -294,6 +308,8 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
     const int n = n_orb, n2 = 2 * n;
     const int nr = bsz(R), ns = bsz(S), np = bsz(P), nq = bsz(Q);
     const bool exch = ax != 0.0 && lc;
+    const CdSrc sR{stk(R), 0, nr, 1, n2, nr}, sS{stk(S), 0, ns, 1, n2, ns};   // [C_B;SC_B]
+    const CdSrc sQ{swp(Q), 0, 1, nq, nq, n2}, sP{swp(P), 0, 1, np, np, n2};   // [SC_B;C_B]^T
     // per product: digit operands (16 bytes per padded element), FP64 results, maxima and exponents
     const long long rV = up_to(ns, 128), rH = up_to(n2, 32), rF = up_to(n2, 128), rG = up_to(nq, 128);
     const long long kV = pad64(nr), kH = pad64(ns), k2 = pad64(n2), ldf = up_to(n2, 4), ldh = up_to(ns, 4);
@@ -326,18 +342,19 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
         cd_max(*this, kc, sV, (int)rV, mV);
         cd_split(*this, kc, sV, oV, mV, eV);
         cd_gemm(*this, TINCR_KF_AO_TRANSFORM, kc, ns, n2, nr, oV, false, cd_stkB(R), true,
-                CdEpiStore{CdScale{eV, eB, (int)rV, 0}, H, n2 * ldh, (int)ldh, ns, n2, mH, (int)rH});
+                CdEpiStore{CdScale{eV, eB, (int)rV, 0, sV, sR}, H, n2 * ldh, (int)ldh, ns, n2, mH, (int)rH});
         if (exch) {
             const DgOperand oH = operand(n2, ns, 5), oF = operand(n2, n2, 7);
-            cd_split(*this, kc, CdSrc{H, n2 * ldh, ldh, 1, n2, ns}, oH, mH, eH);
+            const CdSrc sH{H, n2 * ldh, ldh, 1, n2, ns}, sF{F, n2 * ldf, ldf, 1, n2, n2};
+            cd_split(*this, kc, sH, oH, mH, eH);
             cd_gemm(*this, TINCR_KF_AO_EXCHANGE, kc, n2, n2, ns, cd_stkA(S), true, oH, false,
-                    CdEpiF{CdScale{eA, eH, 0, (int)rH}, F, n2 * ldf, (int)ldf, n, d_glr_ao.p, ax, d3, d2, mF, (int)rF});
+                    CdEpiF{CdScale{eA, eH, 0, (int)rH, sS, sH}, F, n2 * ldf, (int)ldf, n, d_glr_ao.p, ax, d3, d2, mF, (int)rF});
             if (ac != 0.0)
                 launch_coulomb(stream, kc, n, n_atoms, d_ao_off.p, d_gamma.p, d3, d2, nullptr, F, nullptr, ac, ldf,
                                n2 * ldf, mF, (int)rF);
-            cd_split(*this, kc, CdSrc{F, n2 * ldf, ldf, 1, n2, n2}, oF, mF, eF);
+            cd_split(*this, kc, sF, oF, mF, eF);
             cd_gemm(*this, TINCR_KF_AO_EXCHANGE, kc, n2, nq, n2, oF, false, cd_swpT(Q), true,
-                    CdEpiStore{CdScale{eF, eQ, (int)rF, 0}, GT, nq * ldf, (int)ldf, n2, nq, mG, (int)rG});
+                    CdEpiStore{CdScale{eF, eQ, (int)rF, 0, sF, sQ}, GT, nq * ldf, (int)ldf, n2, nq, mG, (int)rG});
         } else {
             dim3 g(ceil_div(2LL * n * 32, 256), kc);
             diag_dots_kernel<<<g, 256, 0, stream>>>(n, ns, H, ldh, n2 * ldh, stk(S), d3, d2);
@@ -349,10 +366,11 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
             count_launch(stream, "cd_scale_rows");
             check_launch("cd_scale_rows");
         }
-        cd_split(*this, kc, CdSrc{GT, nq * ldf, ldf, 1, nq, n2}, oG, mG, eG);
+        const CdSrc sG{GT, nq * ldf, ldf, 1, nq, n2};
+        cd_split(*this, kc, sG, oG, mG, eG);
         const long long o0 = (long long)c0 * np * nq;
         cd_gemm(*this, TINCR_KF_AO_TRANSFORM, kc, nq, np, n2, oG, false, cd_swpT(P), true,
-                CdEpiOut{CdScale{eG, eP, (int)rG, 0}, out + o0, (long long)np * nq, nq, np, d_omega.p,
+                CdEpiOut{CdScale{eG, eP, (int)rG, 0, sG, sP}, out + o0, (long long)np * nq, nq, np, d_omega.p,
                          Xomega ? Xomega + o0 : nullptr, alpha, beta});
     }
     tc_err_watch();   // reported by the next sync()

@@ -31,6 +31,7 @@
 #include "kernels.cuh"
 #include "gemm_f64.cuh"
 #include "ops.cuh"
+#include "fixed8.cuh"
 #include "subspace.cuh"
 #include "tda.cuh"
 
@@ -158,8 +159,8 @@ coulomb_kernel(int n, int n_atoms, const int *__restrict__ ao_off, const double 
             const double f01 = f[(long long)mu * ldf + n + mu] += z;
             const double f10 = f[(long long)(n + mu) * ldf + mu] += z;
             if (fmx) {
-                atomicMax(fmx + (long long)b * fmx_b + mu, (unsigned)__double2hiint(f01) & 0x7fffffffu);
-                atomicMax(fmx + (long long)b * fmx_b + n + mu, (unsigned)__double2hiint(f10) & 0x7fffffffu);
+                atomicMax(fmx + (long long)b * fmx_b + mu, cd_hi_any(f01));
+                atomicMax(fmx + (long long)b * fmx_b + n + mu, cd_hi_any(f10));
             }
         }
     }
