@@ -294,6 +294,11 @@ DgOperand Ctx::cd_swpT(int blk) const {
     return cd_operand(b.p + DG_PLANES * b.rows_pad * b.Kpad, bsz(blk), 2LL * n_orb, 5, 1);
 }
 
+// Bytes of workspace; half of them, what the FP64 tiles take at most (product_chunk), where the workspace has to
+// grow on a device with less than four times as much free.  20 products of (H2O)128 in one chunk (1.3 GB) take
+// 2.82 ms, in two 3.03.
+constexpr long long CD_BUDGET = 1536LL << 20;
+
 // Whether the digit GEMMs beat the FP64 tiles for this contraction.
 bool Ctx::digits_pay(int k, int R, int S, int P, int Q, bool exch) const {
     const double n = n_orb, nr = bsz(R), ns = bsz(S), np = bsz(P), nq = bsz(Q);
@@ -310,13 +315,25 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
     const bool exch = ax != 0.0 && lc;
     const CdSrc sR{stk(R), 0, nr, 1, n2, nr}, sS{stk(S), 0, ns, 1, n2, ns};   // [C_B;SC_B]
     const CdSrc sQ{swp(Q), 0, 1, nq, nq, n2}, sP{swp(P), 0, 1, np, np, n2};   // [SC_B;C_B]^T
-    // per product: digit operands (16 bytes per padded element), FP64 results, maxima and exponents
+    // per product: digit operands (16 bytes per padded element), FP64 results, maxima and exponents.  V, H and G
+    // live one after the other and share their planes, H and G^T their FP64 results; F has its own.
     const long long rV = up_to(ns, 128), rH = up_to(n2, 32), rF = up_to(n2, 128), rG = up_to(nq, 128);
     const long long kV = pad64(nr), kH = pad64(ns), k2 = pad64(n2), ldf = up_to(n2, 4), ldh = up_to(ns, 4);
-    const long long el = rV * kV + (exch ? rH * kH + rF * k2 : 0) + rG * k2;
-    const long long f64 = n2 * ldh + (exch ? n2 * ldf : 0) + nq * ldf + 3LL * n, ints = rV + rH + rF + rG;
+    const long long shared = std::max({rV * kV, exch ? rH * kH : 0LL, rG * k2}), el = shared + (exch ? rF * k2 : 0);
+    const long long hg = std::max(n2 * ldh, nq * ldf), f64 = hg + (exch ? n2 * ldf : 0) + 3LL * n;
+    const long long ints = rV + rH + rF + rG;
     const long long per = el * 16 + f64 * 8 + ints * 8;
-    const int kc_max = (int)std::max<long long>(1, std::min<long long>({(long long)k, 64, ((long long)1536 << 20) / per}));
+    // chunks of equal size
+    auto chunk = [&](long long budget) {
+        const long long most = std::max<long long>(1, std::min<long long>(64, budget / per)), count = (k + most - 1) / most;
+        return (int)((k + count - 1) / count);
+    };
+    int kc_max = chunk(CD_BUDGET);
+    if ((size_t)(DG_PLANES * el * kc_max) > cd_pl.n || (size_t)(f64 * kc_max) > cd_f64.n) {
+        size_t free_bytes = 0, total = 0;
+        TINCR_CUDA(cudaMemGetInfo(&free_bytes, &total));
+        if (free_bytes < 4 * (size_t)CD_BUDGET) kc_max = chunk(CD_BUDGET / 2);
+    }
     cd_pl.reserve((size_t)(DG_PLANES * el * kc_max));
     cd_f64.reserve((size_t)(f64 * kc_max));
     cd_int.reserve((size_t)(2 * ints * kc_max));
@@ -326,13 +343,8 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
         const int kc = std::min(kc_max, k - c0);
         const double *Vc = V + (long long)c0 * nr * ns;
         bf16 *pl = cd_pl.p;
-        auto operand = [&](long long rows, long long K, int rt) {
-            const DgOperand o = cd_operand(pl, rows, K, rt, kc);
-            pl += DG_PLANES * o.rows_pad * o.Kpad;
-            return o;
-        };
-        const DgOperand oV = operand(ns, nr, 7), oG = operand(nq, n2, 7);
-        double *H = cd_f64.p, *GT = H + (long long)kc * n2 * ldh, *d3 = GT + (long long)kc * nq * ldf;
+        const DgOperand oV = cd_operand(pl, ns, nr, 7, kc), oG = cd_operand(pl, nq, n2, 7, kc);
+        double *H = cd_f64.p, *GT = H, *d3 = H + kc * hg;
         double *d2 = d3 + (long long)kc * n, *z = d2 + (long long)kc * n, *F = z + (long long)kc * n;
         unsigned *mV = reinterpret_cast<unsigned *>(cd_int.p), *mH = mV + kc * rV, *mF = mH + kc * rH, *mG = mF + kc * rF;
         int *eV = cd_int.p + kc * ints, *eH = eV + kc * rV, *eF = eH + kc * rH, *eG = eF + kc * rF;
@@ -344,7 +356,7 @@ void Ctx::ao_contract_digits(int k, int R, int S, const double *V, int P, int Q,
         cd_gemm(*this, TINCR_KF_AO_TRANSFORM, kc, ns, n2, nr, oV, false, cd_stkB(R), true,
                 CdEpiStore{CdScale{eV, eB, (int)rV, 0, sV, sR}, H, n2 * ldh, (int)ldh, ns, n2, mH, (int)rH});
         if (exch) {
-            const DgOperand oH = operand(n2, ns, 5), oF = operand(n2, n2, 7);
+            const DgOperand oH = cd_operand(pl, n2, ns, 5, kc), oF = cd_operand(pl + DG_PLANES * kc * shared, n2, n2, 7, kc);
             const CdSrc sH{H, n2 * ldh, ldh, 1, n2, ns}, sF{F, n2 * ldf, ldf, 1, n2, n2};
             cd_split(*this, kc, sH, oH, mH, eH);
             cd_gemm(*this, TINCR_KF_AO_EXCHANGE, kc, n2, n2, ns, cd_stkA(S), true, oH, false,

@@ -696,12 +696,14 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
     const int n = n_orb, o = n_occ, v = n_virt, N = n_atoms;
     const size_t nn = (size_t)n * n;
     // device temporaries: one slot per request, kept by the context (about 30 pairs of cudaMalloc and
-    // cudaFree on each call otherwise, each a device synchronisation)
+    // cudaFree on each call otherwise, each a device synchronisation) but for large systems
+    std::vector<DevBuf<double>> once;
+    std::vector<DevBuf<double>> &slots = 40 * nn * sizeof(double) <= KEPT_BYTES ? gtmp : once;   // at most 36 n x n of them
     size_t slot_no = 0;
     struct Buf { double *p; };
     auto take = [&](size_t count) {
-        if (slot_no == gtmp.size()) gtmp.emplace_back();
-        DevBuf<double> &d = gtmp[slot_no++];
+        if (slot_no == slots.size()) slots.emplace_back();
+        DevBuf<double> &d = slots[slot_no++];
         d.reserve(std::max<size_t>(count, 1));
         return Buf{d.p};
     };

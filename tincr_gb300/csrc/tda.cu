@@ -708,7 +708,7 @@ void Ctx::ao_contract(int k, int R, int S, const double *V, int P, int Q, double
     }
     const int n = n_orb;
     const int nr = bsz(R), ns = bsz(S), np = bsz(P), nq = bsz(Q);
-    const int kc_max = product_chunk();
+    const int kc_max = std::min(k, product_chunk());
     const int wmax = std::max(n_occ, n_virt);
     wsH.reserve((size_t)kc_max * 2 * n * wmax);
     wsG.reserve((size_t)kc_max * 2 * n * wmax);
@@ -774,7 +774,7 @@ void Ctx::qtrans_dev(int k, const double *X, double *y_out) {
         return;
     }
     const int n = n_orb, o = n_occ, v = n_virt;
-    const int kc_max = product_chunk();
+    const int kc_max = std::min(k, product_chunk());
     wsH.reserve((size_t)kc_max * 2 * n * v);
     wsd3.reserve((size_t)kc_max * n);
     wsd2.reserve((size_t)kc_max * n);
@@ -798,13 +798,15 @@ void Ctx::products(int k, const double *X, double *AX, int precision) {
     prec = precision;
     g_launches = 0;
     const size_t len = (size_t)ov * k;
-    px.reserve(3 * len);
+    DevBuf<double> once;
+    DevBuf<double> &buf = 3 * len * sizeof(double) <= KEPT_BYTES ? px : once;
+    buf.reserve(3 * len);
     px_bad.reserve(1);
-    double *dXin = px.p, *dX = dXin + len, *dAX = dX + len;
+    double *dXin = buf.p, *dX = dXin + len, *dAX = dX + len;
     int bad = 0;
     // X is checked for non-finite values by the transposition that reads it: the host's pass over 20
     // vectors of (H2O)128 (21 MB) took 1.2 ms of a 2.5 ms call, allocating and freeing the three
-    // buffers on each call 0.2 ms
+    // buffers on each call 0.2 ms (large ones are)
     TINCR_CUDA(cudaMemsetAsync(px_bad.p, 0, sizeof(int), stream));
     TINCR_CUDA(cudaMemcpyAsync(dXin, X, len * sizeof(double), cudaMemcpyHostToDevice, stream));
     TINCR_CUDA(cudaEventRecord(ev0, stream));

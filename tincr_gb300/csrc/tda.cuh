@@ -38,6 +38,9 @@ constexpr double MIXED_TOL_FLOOR = 1e-6;
 // without exchange (H2O)64 1 vector, 50e6: 109 / 135.
 constexpr double CD_MIN_MAC = 45e6;
 
+// Device buffers that only save their allocation are kept between calls up to this size.
+constexpr size_t KEPT_BYTES = (size_t)256 << 20;
+
 struct DgOperand;                      // digit planes of a GEMM operand (digits.cuh)
 struct BatchWork;                      // batched LE / CT TDA workspace (batch.cu)
 void release_batch(BatchWork *w);
@@ -97,7 +100,7 @@ struct Ctx {
     DevBuf<int> d_kind_z, d_kind_norb, d_kind_l, d_kind_m, d_rep_nt;
     DevBuf<double> d_sigma, d_knots, d_coef, d_rep_knots, d_rep_coef, d_rep_dmax;
     DevBuf<double> gw, gv, gcg;            // gradient workspaces
-    std::vector<DevBuf<double>> gtmp;      // its temporaries, by order of request
+    std::vector<DevBuf<double>> gtmp;      // its temporaries, by order of request (up to KEPT_BYTES)
     int last_cg_status = TINCR_OK;
 
     int prec = TINCR_PREC_FP64;           // arithmetic of the contractions in ao_contract
@@ -119,7 +122,7 @@ struct Ctx {
     void tc_err_watch();                  // queue the copy of d_tc_err to h_tc_err (checked at the next sync)
 
     // product workspace
-    DevBuf<double> px;                     // X as given, transposed, A.X of the last tincr_tda_products call
+    DevBuf<double> px;                     // X as given, transposed, A.X of the last tincr_tda_products call (up to KEPT_BYTES)
     DevBuf<int> px_bad;
     DevBuf<double> wsH, wsF, wsG, wsd3, wsd2, wsz;
     // Davidson state
