@@ -239,8 +239,6 @@ inline int f64_tile_for(int M, int N, long long z, int n_sm) {
     return tm[best];
 }
 
-constexpr int F64_SMS = 152;   // SMs of a GB300, for the choice of the tile
-
 // Launch helper.  splitk > 1 requires an accumulating epilogue.
 template <class W, bool TA, bool TB, class Epi>
 void gemm_f64_launch(cudaStream_t st, int M, int N, int K, int k_chunk, int splitk, const double *A, int lda,
@@ -252,7 +250,7 @@ void gemm_f64_launch(cudaStream_t st, int M, int N, int K, int k_chunk, int spli
 }
 
 template <bool TA, bool TB, class Epi>
-void gemm_f64(cudaStream_t st, int M, int N, int K, const double *A, int lda, long long sA,
+void gemm_f64(cudaStream_t st, int n_sm, int M, int N, int K, const double *A, int lda, long long sA,
               const double *B, int ldb, long long sB, int batch, Epi epi, int splitk = 1) {
     if (M <= 0 || N <= 0 || batch <= 0) return;
     if (splitk < 1) splitk = 1;
@@ -264,7 +262,7 @@ void gemm_f64(cudaStream_t st, int M, int N, int K, const double *A, int lda, lo
     auto go = [&](auto w) {
         gemm_f64_launch<decltype(w), TA, TB>(st, M, N, K, k_chunk, splitk, A, lda, sA, B, ldb, sB, batch, epi);
     };
-    switch (f64_tile_for(M, N, (long long)batch * splitk, F64_SMS)) {
+    switch (f64_tile_for(M, N, (long long)batch * splitk, n_sm)) {
         case 64: go(F64T64{}); break;
         case 32: go(F64T32{}); break;
         case 16: go(F64T16{}); break;

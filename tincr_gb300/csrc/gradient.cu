@@ -551,10 +551,10 @@ void Ctx::plr_adjoint(const double *v, const double *Y, double scale_p, double s
         }
         int slot = prof_begin(TINCR_KF_GRADIENT);
         EpiStore e{C, 0, n, alpha, beta};
-        if (!ta && !tb) gemm_f64<false, false>(stream, n, n, n, A, n, 0, B, n, 0, 1, e);
-        else if (ta && !tb) gemm_f64<true, false>(stream, n, n, n, A, n, 0, B, n, 0, 1, e);
-        else if (!ta && tb) gemm_f64<false, true>(stream, n, n, n, A, n, 0, B, n, 0, 1, e);
-        else gemm_f64<true, true>(stream, n, n, n, A, n, 0, B, n, 0, 1, e);
+        if (!ta && !tb) gemm_f64<false, false>(stream, n_sm, n, n, n, A, n, 0, B, n, 0, 1, e);
+        else if (ta && !tb) gemm_f64<true, false>(stream, n_sm, n, n, n, A, n, 0, B, n, 0, 1, e);
+        else if (!ta && tb) gemm_f64<false, true>(stream, n_sm, n, n, n, A, n, 0, B, n, 0, 1, e);
+        else gemm_f64<true, true>(stream, n_sm, n, n, n, A, n, 0, B, n, 0, 1, e);
         prof_end(slot, 2.0 * n * (double)n * n, 24.0 * nn);
     };
     mm(false, false, s, v, sv, 1.0, 0.0);        // s v
@@ -761,10 +761,10 @@ int Ctx::gradient(const int *atom_kind, double r_lr_, const double *P, const dou
         }
         EpiStore e{C, 0, ldc, alpha, beta};
         int slot = prof_begin(TINCR_KF_GRADIENT);
-        if (!ta && !tb) gemm_f64<false, false>(stream, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
-        else if (ta && !tb) gemm_f64<true, false>(stream, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
-        else if (!ta && tb) gemm_f64<false, true>(stream, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
-        else gemm_f64<true, true>(stream, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
+        if (!ta && !tb) gemm_f64<false, false>(stream, n_sm, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
+        else if (ta && !tb) gemm_f64<true, false>(stream, n_sm, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
+        else if (!ta && tb) gemm_f64<false, true>(stream, n_sm, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
+        else gemm_f64<true, true>(stream, n_sm, M, Nn, K, A, lda, 0, B, ldb, 0, 1, e);
         prof_end(slot, 2.0 * M * (double)Nn * K, 8.0 * ((double)M * K + (double)K * Nn + (double)M * Nn));
     };
 

@@ -96,9 +96,9 @@ void products_noalloc(Ctx &c, int k, const double *X, double *AX) {
         const double *xb = X + (long long)b * ov;
         double *ab = AX + (long long)b * ov;
         // H = [Co; SCo] X
-        gemm_f64<false, false>(st, 2 * n, v, o, c.dLst.p, o, 0, xb, v, 0, 1, EpiStore{H, 0, v, 1.0, 0.0});
+        gemm_f64<false, false>(st, c.n_sm, 2 * n, v, o, c.dLst.p, o, 0, xb, v, 0, 1, EpiStore{H, 0, v, 1.0, 0.0});
         if (c.lc) {
-            gemm_f64<false, true>(st, 2 * n, 2 * n, v, H, v, 0, c.dRv.p, v, 0, 1,
+            gemm_f64<false, true>(st, c.n_sm, 2 * n, 2 * n, v, H, v, 0, c.dRv.p, v, 0, 1,
                                   EpiLcHadamard{F, c.d_glr_ao.p, d3, d2, n, -0.25});
         } else {
             dim3 g(ceil_div(2LL * n * 32, 256), 1);
@@ -108,14 +108,14 @@ void products_noalloc(Ctx &c, int k, const double *X, double *AX) {
         launch_coulomb(st, 1, n, c.n_atoms, c.d_ao_off.p, c.d_gamma.p, d3, d2, c.lc ? nullptr : z, c.lc ? F : nullptr,
                        nullptr, 1.0);
         if (c.lc) {
-            gemm_f64<false, false>(st, 2 * n, v, 2 * n, F, 2 * n, 0, c.dRsw.p, v, 0, 1, EpiStore{G, 0, v, 1.0, 0.0});
+            gemm_f64<false, false>(st, c.n_sm, 2 * n, v, 2 * n, F, 2 * n, 0, c.dRsw.p, v, 0, 1, EpiStore{G, 0, v, 1.0, 0.0});
         } else {
             dim3 g(ceil_div(2LL * n * v, 256), 1);
             scale_rows_kernel<<<g, 256, 0, st>>>(n, v, z, c.dRv.p, G);
             check_launch("scale_rows");
         }
         // AX = omega o X + [SCo; Co]^T G
-        gemm_f64<true, false>(st, o, v, 2 * n, c.dLsw.p, o, 0, G, v, 0, 1, EpiOmega{ab, c.d_omega.p, xb, ov, v});
+        gemm_f64<true, false>(st, c.n_sm, o, v, 2 * n, c.dLsw.p, o, 0, G, v, 0, 1, EpiOmega{ab, c.d_omega.p, xb, ov, v});
     }
     c.sync();
 }

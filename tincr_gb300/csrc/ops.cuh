@@ -53,7 +53,7 @@ template <bool TA, bool TB, class Epi>
 static void pgemm(Ctx &c, int family, int M, int N, int K, const double *A, int lda, long long sA, const double *B,
                   int ldb, long long sB, int batch, Epi epi, int splitk = 1) {
     int slot = c.prof_begin(family);
-    gemm_f64<TA, TB>(c.stream, M, N, K, A, lda, sA, B, ldb, sB, batch, epi, splitk);
+    gemm_f64<TA, TB>(c.stream, c.n_sm, M, N, K, A, lda, sA, B, ldb, sB, batch, epi, splitk);
     double nb = (double)batch;
     double bytes = 8.0 * ((double)M * K * (sA ? nb : 1.0) + (double)K * N * (sB ? nb : 1.0) + (double)M * N * nb);
     c.prof_end(slot, 2.0 * M * (double)N * K * nb, bytes);

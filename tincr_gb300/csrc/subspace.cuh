@@ -21,7 +21,6 @@
 namespace tincr {
 
 constexpr int SK_ROWS = 32, SK_COLS = 64, SK_T = 256;
-constexpr int SK_FULL = 152;   // SMs of a GB300
 
 // out[x chunk][M x nb] = A[M x L] . B[nb x L]^T over the chunk, leading dimension ld; rows of B at or
 // beyond nb are read as zero.
@@ -180,10 +179,10 @@ inline void skinny_dots(cudaStream_t st, int n_sm, int M, int nb, long long L, c
 }
 
 template <class Epi>
-inline void skinny_comb(cudaStream_t st, int rows, int m, long long L, const double *Y, long long ysr, long long ysi,
+inline void skinny_comb(cudaStream_t st, int n_sm, int rows, int m, long long L, const double *Y, long long ysr, long long ysi,
                         const double *V, long long ldv, Epi epi) {
     if (rows <= 0 || L <= 0) return;
-    if ((L + SK_T - 1) / SK_T < SK_FULL) {   // fewer CTAs of 256 columns than SMs
+    if ((L + SK_T - 1) / SK_T < n_sm) {   // fewer CTAs of 256 columns than SMs
         skinny_comb_kernel<4, Epi><<<dim3((unsigned)((L + 63) / 64), (unsigned)((rows + 3) / 4)), 64, 0, st>>>(m, L, Y, ysr, ysi,
                                                                                                          V, ldv, rows, epi);
         count_launch(st, "skinny_comb");

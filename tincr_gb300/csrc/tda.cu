@@ -584,7 +584,7 @@ void Ctx::upload_mo(int n, const double *C, const double *S) {
     upload(stream, dC, C, (size_t)n * n);
     upload(stream, dS_, S, (size_t)n * n);
     dSC.alloc((size_t)n * n);
-    gemm_f64<false, false>(stream, n, n, n, dS_.p, n, 0, dC.p, n, 0, 1, EpiStore{dSC.p, 0, n, 1.0, 0.0});
+    gemm_f64<false, false>(stream, n_sm, n, n, n, dS_.p, n, 0, dC.p, n, 0, 1, EpiStore{dSC.p, 0, n, 1.0, 0.0});
     sync();
 }
 
@@ -780,7 +780,7 @@ void Ctx::qtrans_dev(int k, const double *X, double *y_out) {
     wsd2.reserve((size_t)kc_max * n);
     for (int c0 = 0; c0 < k; c0 += kc_max) {
         int kc = std::min(kc_max, k - c0);
-        gemm_f64<false, false>(stream, 2 * n, v, o, dLst.p, o, 0, X + (long long)c0 * ov, v, ov, kc,
+        gemm_f64<false, false>(stream, n_sm, 2 * n, v, o, dLst.p, o, 0, X + (long long)c0 * ov, v, ov, kc,
                                EpiStore{wsH.p, 2LL * n * v, v, 1.0, 0.0});
         dim3 g(ceil_div(2LL * n * 32, 256), kc);
         diag_dots_kernel<<<g, 256, 0, stream>>>(n, v, wsH.p, v, 2LL * n * v, dRv.p, wsd3.p, wsd2.p);
@@ -957,8 +957,8 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
             dg_ritz(n_roots, m, dYt.p, dR.p, dRk.p, du.p);
         } else if (n_roots <= 32) {
             int slot = prof_begin(TINCR_KF_SUBSPACE);
-            skinny_comb(stream, n_roots, m, ov, dYt.p, m, 1, dV.p, ov, CombStore{dR.p, ov, 1.0, 0.0});
-            skinny_comb(stream, n_roots, m, ov, dYt.p, m, 1, dAV.p, ov, CombResidual{dRk.p, dR.p, du.p, ov});
+            skinny_comb(stream, n_sm, n_roots, m, ov, dYt.p, m, 1, dV.p, ov, CombStore{dR.p, ov, 1.0, 0.0});
+            skinny_comb(stream, n_sm, n_roots, m, ov, dYt.p, m, 1, dAV.p, ov, CombResidual{dRk.p, dR.p, du.p, ov});
             prof_end(slot, 4.0 * n_roots * (double)m * ov, 8.0 * (2.0 * m + 3.0 * n_roots) * ov);
         } else {
             pgemm<false, false>(*this, TINCR_KF_SUBSPACE, n_roots, (int)ov, m, dYt.p, m, 0, dV.p, (int)ov, 0, 1,
@@ -1014,7 +1014,7 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                     // c = V T^T  [m x kadd];  T -= c^T V
                     int slot = prof_begin(TINCR_KF_SUBSPACE);
                     skinny_dots(stream, n_sm, m, kadd, ov, dV.p, ov, dT.p, ov, dc.p, kadd, sk_part);
-                    skinny_comb(stream, kadd, m, ov, dc.p, 1, kadd, dV.p, ov, CombStore{dT.p, ov, -1.0, 1.0});
+                    skinny_comb(stream, n_sm, kadd, m, ov, dc.p, 1, kadd, dV.p, ov, CombStore{dT.p, ov, -1.0, 1.0});
                     prof_end(slot, 4.0 * kadd * (double)m * ov, 8.0 * (2.0 * m + 3.0 * kadd) * ov);
                 } else {
                     TINCR_CUDA(cudaMemsetAsync(dc.p, 0, (size_t)kadd * m * sizeof(double), stream));
@@ -1058,7 +1058,7 @@ int Ctx::davidson(int n_roots, int max_iter, double tol, bool from_ritz, std::ve
                             // c = Q t  [acc x 1] over the vectors accepted in this step;  t -= c^T Q
                             int slot = prof_begin(TINCR_KF_SUBSPACE);
                             skinny_dots(stream, n_sm, acc, 1, ov, dV.p + (long long)m0 * ov, ov, t, ov, dc.p, 1, sk_part);
-                            skinny_comb(stream, 1, acc, ov, dc.p, acc, 1, dV.p + (long long)m0 * ov, ov,
+                            skinny_comb(stream, n_sm, 1, acc, ov, dc.p, acc, 1, dV.p + (long long)m0 * ov, ov,
                                         CombStore{t, ov, -1.0, 1.0});
                             prof_end(slot, 4.0 * acc * (double)ov, 8.0 * (acc + 2.0) * ov);
                         }
