@@ -48,73 +48,6 @@ struct EpiAtomicAdd {
     }
 };
 
-// One 64 x 64 output tile over k in [kbeg, kend): acc[i][j] holds C(m0 + ty + 16 i, n0 + tx + 16 j)
-// for thread (tx, ty) = (tid & 15, tid >> 4).  All 256 threads of the CTA take part.
-template <bool TA, bool TB>
-__device__ __forceinline__ void gemm_f64_tile(int M, int N, int kbeg, int kend, const double *__restrict__ A, int lda,
-                                              const double *__restrict__ B, int ldb, int m0, int n0,
-                                              double (&As)[GB_K][GB_M + 1], double (&Bs)[GB_K][GB_N + 1],
-                                              double (&acc)[4][4]) {
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-
-    double ra[4], rb[4];
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int m, k;
-            if (!TA) { m = tid >> 2; k = ((tid & 3) << 2) + e; }
-            else     { k = tid >> 4; m = ((tid & 15) << 2) + e; }
-            int gm = m0 + m, gk = k0 + k;
-            ra[e] = (gm < M && gk < kend) ? (TA ? A[(long long)gk * lda + gm] : A[(long long)gm * lda + gk]) : 0.0;
-            int n, kb;
-            if (!TB) { kb = tid >> 4; n = ((tid & 15) << 2) + e; }
-            else     { n = tid >> 2; kb = ((tid & 3) << 2) + e; }
-            int gn = n0 + n, gkb = k0 + kb;
-            rb[e] = (gn < N && gkb < kend) ? (TB ? B[(long long)gn * ldb + gkb] : B[(long long)gkb * ldb + gn]) : 0.0;
-        }
-    };
-    auto store = [&]() {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int m, k;
-            if (!TA) { m = tid >> 2; k = ((tid & 3) << 2) + e; }
-            else     { k = tid >> 4; m = ((tid & 15) << 2) + e; }
-            As[k][m] = ra[e];
-            int n, kb;
-            if (!TB) { kb = tid >> 4; n = ((tid & 15) << 2) + e; }
-            else     { n = tid >> 2; kb = ((tid & 3) << 2) + e; }
-            Bs[kb][n] = rb[e];
-        }
-    };
-
-    if (kbeg < kend) {
-        load(kbeg);
-        for (int k0 = kbeg; k0 < kend; k0 += GB_K) {
-            __syncthreads();
-            store();
-            __syncthreads();
-            if (k0 + GB_K < kend) load(k0 + GB_K);
-#pragma unroll
-            for (int kk = 0; kk < GB_K; ++kk) {
-                double a[4], b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-            }
-        }
-    }
-}
-
 // Tile of TM x TN outputs by TY x TX threads, KS deep slices.
 template <int TY, int TX, int R, int KS_>
 struct F64Tile {

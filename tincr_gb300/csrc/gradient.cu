@@ -340,7 +340,7 @@ struct PairArgs {
 // centre 1, q of centre 2; r = the vector from centre 1 to 2, u = r / |r|), summed over the block before
 // anything is differentiated: with w's s-s entry a, its s-p and p-s vectors b and c, its p-p matrix m,
 //     sum_pq w_pq M_pq = a V0 + (b.u) V1 + (c.u) V2 + (u m u) (V4 - V3) + tr(m) V3
-// in the integrals V of sk_element's slot order, whose gradient needs no angular factors per element.
+// in the integrals V of sk_value's slot order, whose gradient needs no angular factors per element.
 __device__ __forceinline__ void sk_contract(const PairArgs &a, int k1, int k2, int n1, int n2, const double *W,
                                             const double *cf, const double N3[4], const double fd[3], const double u[3],
                                             double r, double g[3]) {

@@ -87,49 +87,8 @@ TINCR_HD void bspline3_eval(const double *t, const double *c, int l, const doubl
 // Cartesian axis of a real p orbital: m = -1 -> y (1), 0 -> z (2), +1 -> x (0)
 TINCR_HD int p_axis(int m) { return m == -1 ? 1 : (m == 0 ? 2 : 0); }
 
-// Value of one SK matrix element and its gradient w.r.t. r (vector from centre 1 to 2).
-// u: direction cosines, r: distance, v/dv: integrals and r-derivatives in slot order.
-TINCR_HD void sk_element(int l1, int m1, int l2, int m2, const double u[3], double r, const double v[SK_SLOTS],
-                         const double dv[SK_SLOTS], double &val, double g[3]) {
-    // angular factors: up to two terms (slot, P, grad_u P)
-    int slot[2];
-    double P[2];
-    double gu[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    int nt = 0;
-    if (l1 == 0 && l2 == 0) {
-        slot[0] = 0; P[0] = 1.0; nt = 1;
-    } else if (l1 == 0 && l2 == 1) {
-        int c = p_axis(m2);
-        slot[0] = 1; P[0] = u[c]; gu[0][c] = 1.0; nt = 1;
-    } else if (l1 == 1 && l2 == 0) {
-        int c = p_axis(m1);
-        slot[0] = 2; P[0] = u[c]; gu[0][c] = 1.0; nt = 1;
-    } else {
-        int c1 = p_axis(m1), c2 = p_axis(m2);
-        if (c1 == c2) {
-            int o0 = (c1 + 1) % 3, o1 = (c1 + 2) % 3;
-            if (o0 > o1) { int tmp = o0; o0 = o1; o1 = tmp; }
-            slot[0] = 3; P[0] = u[o0] * u[o0] + u[o1] * u[o1];
-            gu[0][o0] = 2.0 * u[o0]; gu[0][o1] = 2.0 * u[o1];
-            slot[1] = 4; P[1] = u[c1] * u[c1]; gu[1][c1] = 2.0 * u[c1];
-        } else {
-            double p = u[c1] * u[c2];
-            slot[0] = 3; P[0] = -p; gu[0][c1] = -u[c2]; gu[0][c2] = -u[c1];
-            slot[1] = 4; P[1] = p; gu[1][c1] = u[c2]; gu[1][c2] = u[c1];
-        }
-        nt = 2;
-    }
-    val = 0.0;
-    g[0] = g[1] = g[2] = 0.0;
-    for (int t = 0; t < nt; ++t) {
-        double V = v[slot[t]], dV = dv[slot[t]];
-        val += P[t] * V;
-        double gdotu = gu[t][0] * u[0] + gu[t][1] * u[1] + gu[t][2] * u[2];
-        for (int c = 0; c < 3; ++c) g[c] += (gu[t][c] - gdotu * u[c]) * V / r + P[t] * dV * u[c];
-    }
-}
-
-// Value of one SK matrix element (the value part of sk_element).
+// Value of one SK matrix element; u: direction cosines from centre 1 to 2, v: integrals in slot order (0 s-s,
+// 1 s-p, 2 p-s, 3 p-p pi, 4 p-p sigma).
 TINCR_HD double sk_value(int l1, int m1, int l2, int m2, const double u[3], const double v[SK_SLOTS]) {
     if (l1 == 0 && l2 == 0) return v[0];
     if (l1 == 0) return u[p_axis(m2)] * v[1];
