@@ -59,3 +59,16 @@ def test_a_full_gpu_of_small_systems_takes_about_the_time_of_one(gpu_ctx, name):
             t.append(gscc.last_ms(gpu_ctx))
         ms[count] = min(t)
     assert ms[304] < 1.8 * ms[1], ms
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 40, 310])
+@pytest.mark.parametrize("name", ["h2", "water2", "acene1", "acene3"])
+def test_scc_fp32_start_of_small_systems(gpu_ctx, name, count):
+    ref = _systems(name, True)
+    got, rc = gscc.scc_batch(gpu_ctx, [ref[i % 4][0] for i in range(count)], tol=1e-11, fp32_start=True)
+    assert rc == _lib.OK
+    for i, g in enumerate(got):
+        h = ref[i % 4][1]
+        assert abs(g.energy - h.energy) < 1e-11
+        assert np.max(np.abs(g.p - h.p)) < 1e-9
