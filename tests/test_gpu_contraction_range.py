@@ -50,7 +50,9 @@ def test_products_up_to_the_largest_double(n, o, v, k, lc):
     assert np.array_equal(es.compute_products(np.ldexp(x, p)), np.ldexp(y, p))
     assert np.frexp(np.abs(np.ldexp(y, p)).max())[1] == 1024
     for p in range(1025 - top, 1025 - top + 40, 3):
-        got, want = es.compute_products(np.ldexp(x, min(p, 1020))), np.ldexp(y, min(p, 1020))
+        got = es.compute_products(np.ldexp(x, min(p, 1020)))
+        with np.errstate(over="ignore"):
+            want = np.ldexp(y, min(p, 1020))
         # what is out of range is not finite, what is finite is right
         assert not np.any(np.isfinite(got) & ~np.isfinite(want))
         fine = np.isfinite(got)

@@ -1,5 +1,6 @@
 """A.X of an X that is not finite: refused with the status, A.X left as it was, and the context right afterwards,
-in both precisions and on both sides of the number of multiply-adds from which FP64 runs on digits."""
+in both precisions, on both sides of the number of multiply-adds from which FP64 runs on digits and of the 8192
+values from which the device checks X."""
 
 import numpy as np
 import pytest
@@ -9,7 +10,7 @@ from tincr_gb300 import tda as T
 from tincr_gb300._lib import dptr
 from test_gpu_product_sizes import _system
 
-SIZES = [(33, 16, 17, 1), (33, 16, 17, 3), (128, 64, 64, 24)]
+SIZES = [(33, 16, 17, 1), (33, 16, 17, 3), (128, 64, 64, 2), (128, 64, 64, 3), (128, 64, 64, 24)]
 
 
 @pytest.mark.gpu

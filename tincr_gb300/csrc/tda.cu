@@ -804,19 +804,24 @@ void Ctx::products(int k, const double *X, double *AX, int precision) {
     px_bad.reserve(1);
     double *dXin = buf.p, *dX = dXin + len, *dAX = dX + len;
     int bad = 0;
-    // X is checked for non-finite values by the transposition that reads it: the host's pass over 20
-    // vectors of (H2O)128 (21 MB) took 1.2 ms of a 2.5 ms call, allocating and freeing the three
-    // buffers on each call 0.2 ms (large ones are)
-    TINCR_CUDA(cudaMemsetAsync(px_bad.p, 0, sizeof(int), stream));
+    // Beyond a few thousand values X is checked for non-finite ones by the transposition that reads it: the
+    // host's pass over 20 vectors of (H2O)128 (21 MB) took 1.2 ms of a 2.5 ms call, allocating and freeing the
+    // three buffers on each call 0.2 ms (large ones are).  A short X the host checks faster than the flag comes
+    // back: 225 values (benzene, FP64) 60 against 71 us, 8064 (naphthalene) 87 against 96, 13500 level.
+    const bool on_device = len > 8192;
+    if (on_device) TINCR_CUDA(cudaMemsetAsync(px_bad.p, 0, sizeof(int), stream));
+    else check_finite(X, len, "X");
     TINCR_CUDA(cudaMemcpyAsync(dXin, X, len * sizeof(double), cudaMemcpyHostToDevice, stream));
     TINCR_CUDA(cudaEventRecord(ev0, stream));
-    launch_transpose((int)ov, k, dXin, dX, px_bad.p);     // [ov x k] -> [k x ov]
+    launch_transpose((int)ov, k, dXin, dX, on_device ? px_bad.p : nullptr);   // [ov x k] -> [k x ov]
     products_dev(k, dX, dAX, nullptr);
     launch_transpose(k, (int)ov, dAX, dXin);              // back to [ov x k]
     TINCR_CUDA(cudaEventRecord(ev1, stream));
-    TINCR_CUDA(cudaMemcpyAsync(&bad, px_bad.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    sync();
-    if (bad) fail(TINCR_NONFINITE, "non-finite value in X");
+    if (on_device) {
+        TINCR_CUDA(cudaMemcpyAsync(&bad, px_bad.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        sync();
+        if (bad) fail(TINCR_NONFINITE, "non-finite value in X");
+    }
     TINCR_CUDA(cudaMemcpyAsync(AX, dXin, (size_t)ov * k * sizeof(double), cudaMemcpyDeviceToHost, stream));
     sync();
     float ms = 0.f;
