@@ -54,6 +54,23 @@ def test_scc_of_degenerate_frontier_levels(gpu_ctx, rings, count, lc, gap):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 160])
+def test_missing_gap_is_not_searched_for_in_every_iteration(gpu_ctx, count):
+    """Forty iterations (the tolerance is out of reach) without a gap cost about as much as their eigenpairs, less
+    than 2.3 times the purifications with a gap here; both in each were about three times them."""
+    ms = {}
+    for gap in (0.0, 0.3):
+        sy, given, _ = _degenerate(4, False, gap, 5)
+        t = []
+        for _ in range(5):
+            got, rc = gscc.scc_batch(gpu_ctx, [sy] * count, tol=1e-300, given=[given] * count, max_iter=40)
+            assert rc == _lib.NOT_CONVERGED and got[0].iterations == 40
+            t.append(gscc.last_ms(gpu_ctx))
+        ms[gap] = min(t)
+    assert ms[0.0] < 2.7 * ms[0.3], ms
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("lc", [True, False])
 def test_scc_of_two_separate_atoms(gpu_ctx, lc):
     """Two H atoms out of range of each other: one level of two is filled whichever the eigensolver takes, so

@@ -1304,6 +1304,10 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
     // P' = S^1/2 P S^1/2 of the starting density
     gemm<T>(n, n, n, T(1), w.Sh, n, false, w.P, n, false, T(0), w.T1, n, sm);
     gemm_sym<T>(n, n, T(1), w.T1, n, false, w.Sh, n, false, T(0), w.Pp, n, sm);
+    // a matrix without a gap costs all steps of the purification and the eigenpairs too, and often stays so: after
+    // each failure in a row twice as many iterations (32 at most) go to the eigenpairs at once (77 stacked
+    // anthracene dimers without LC, three of which never converge: 1357 -> 873 ms, 2047 with the eigenpairs alone)
+    int failed = 0, wait = 0;
     for (int k = 0; k < limit; ++k) {
         ++st.it;
         sc_charges<T>(n, N, w.P, w.S, w.gam, p0, sm);
@@ -1374,12 +1378,18 @@ __device__ void sc_iterate(const ScArgs &a, const tincr_scc_system &sy, const Sc
         sc_bar(sm);
         if constexpr (sizeof(T) == 8) {
             // P' = 2 X, P = X_orth P' X_orth with X_orth = S^-1/2
-            if (sc_purify(n, o, w.EA, w.Pp, w.T1, w.dg, sm)) {
+            if (wait > 0) {
+                --wait;
+            } else if (sc_purify(n, o, w.EA, w.Pp, w.T1, w.dg, sm)) {
+                failed = 0;
                 SC_FOR(t, nn) w.Pp[t] *= T(2);
                 sc_bar(sm);
                 sc_prod(w.dg, n, n, n, T(1), OP_X, w.X, n, false, OP_ANY, w.Pp, n, false, T(0), w.T1, n, false, sm);
                 sc_prod(w.dg, n, n, n, T(1), OP_ANY, w.T1, n, false, OP_X, w.X, n, false, T(0), w.P, n, true, sm);
                 continue;
+            } else {
+                wait = 1 << failed;
+                if (failed < 5) ++failed;
             }
         }
         if (!sc_eigh<T>(n, o, w.EA, w.Z, w.W, piv, w.dg, sm)) {
