@@ -68,7 +68,7 @@ constexpr int SC_SLOTS_PER_SM = 2;
 constexpr int SC_KS = 32;              // k depth of a GEMM slice
 constexpr int SC_DIGITS = 20000;       // n^3 per CTA from which the iterations' FP64 products run on digits
 constexpr int SC_CMAX = 16;            // CTAs per cluster
-constexpr int SC_FILL = 4;             // CTAs per SM that a batch of large systems is spread over (twice those that run at once)
+constexpr double SC_FILL = 4.0;        // CTAs per SM that a batch of large systems is spread over (twice those that run at once)
 constexpr double SC_SMALL = 96.0;      // orbitals below which systems count as small (sc_ctas_per_system)
 
 struct ScArgs {
@@ -1581,7 +1581,9 @@ __global__ void __launch_bounds__(SC_T, SC_SLOTS_PER_SM) scc_kernel(ScArgs a) {
 // iteration (a few large systems decide, a few large ones among thousands of small ones do not).  Below 16
 // orbitals a second CTA only adds barriers; below SC_SMALL the systems of a batch converge alike, so more
 // than what runs at once is a second wave, while the larger ones (dimers) differ by hundreds of iterations
-// and the last ones are worth the CTAs.  Clusters of 16 fit on a GPC a few at a time, so small systems take
+// and the last ones are worth the CTAs; up to 112 orbitals short of a full second wave (152 pentacenes without
+// LC on 4 CTAs 78.8 ms, on 2 49.6; from the FP32 start 73.7 and 43.9, 68.4 with one CTA and the eigensolver;
+// 152 stacked naphthalene dimers 542 and 582).  Clusters of 16 fit on a GPC a few at a time, so small systems take
 // them up to four.  Kernel time (ms, LC, to 1e-10) with one CTA and the eigensolver in every iteration / two
 // CTAs and more, SC_FILL CTAs per SM for all / this rule:
 //     304 systems of 6 orbitals  1.74 / 3.89 / 1.51     304 of 30 orbitals  11.5 / 16.5 /  8.1
@@ -1597,10 +1599,10 @@ int sc_ctas_per_system(int n_sys, const tincr_scc_system *sys, int n_sm) {
     }
     const double size = w4 / w3;
     const bool small = size < SC_SMALL;
-    const int fill = size < 32.0 ? 1 : small ? 2 : SC_FILL;
+    const double fill = size < 32.0 ? 1.0 : small ? 2.0 : size < 112.0 ? 3.5 : SC_FILL;
     const int most = size < 16.0 ? 1 : size < 32.0 ? 4 : small && n_sys > 4 ? 8 : SC_CMAX;
     int csize = small ? 1 : 2;
-    while (csize < most && 2LL * csize * n_sys <= (long long)fill * n_sm) csize *= 2;
+    while (csize < most && 2.0 * csize * n_sys <= fill * n_sm) csize *= 2;
     return csize;
 }
 
