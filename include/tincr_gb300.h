@@ -38,7 +38,13 @@ typedef enum {
  * ends with FP64 Davidson iterations started from the mixed Ritz vectors (usually one
  * Rayleigh-Ritz step), so the convergence test and the energies are then those of FP64.
  * Setting the environment variable TINCR_GB300_PLANE_GEMM=mma before tincr_ctx_create selects
- * the warp-MMA implementation of the single-system plane GEMM instead of tcgen05. */
+ * the warp-MMA implementation of the single-system plane GEMM instead of tcgen05.
+ *
+ * TINCR_PREC_FP64: contractions of 45e6 multiply-adds and more (all vectors of a call) run as exact
+ * fixed-point digit products on the tensor cores: values to 2^-62 of the largest of their row, sums
+ * exact, one rounding; in the norm as accurate as FP64 sums.  Components some 2^50 below the
+ * largest keep fewer digits than FP64 sums leave them; TINCR_GB300_CONTRACTION=fp64, set before
+ * tincr_ctx_create, keeps all contractions on FP64 instructions. */
 typedef enum {
     TINCR_PREC_FP64 = 0,      /* plain FP64 drop-in                                             */
     TINCR_PREC_BF16X3 = 1     /* three-plane split-BF16 tensor-core products, FP64 subspace       */
@@ -364,7 +370,8 @@ int tincr_rpa_solve(tincr_ctx *ctx, int n_roots, int max_iter, double tol, doubl
 typedef enum {
     TINCR_SCC_LC = 1,              /* long-range corrected (gamma_lr with radius r_lr)                 */
     TINCR_SCC_SK_EXTRAPOLATE = 2,  /* SK splines beyond their grid: boundary polynomial, not zero      */
-    TINCR_SCC_FP32_START = 4       /* FP32 iterations until the commutator is below 1e-5, then FP64    */
+    TINCR_SCC_FP32_START = 4       /* FP32 iterations until the commutator is below 1e-5, then FP64;   */
+                                   /* no gain on 64 acenes, 7 % slower on 529 acene dimers              */
 } tincr_scc_flags;
 
 /* One system of a batched SCC.  Offsets index the packed arrays of tincr_scc_batch. */

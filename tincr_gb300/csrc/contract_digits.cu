@@ -17,8 +17,14 @@
 // The digits are those of fixed8.cuh.  (Digits of 7 bits with x's sign, which truncate towards zero, gave
 // A.X errors 3 to 6 times those of the FP64 FMAs.)
 //
-// Error of A.X against quad precision, digits / FP64 tiles (naphthalene .. decacene, (H2O)16, (H2O)40,
-// C20H22): 7.1e-17 .. 8.5e-17 / 7.3e-17 .. 1.0e-16, the digits below the tiles in every case.
+// Precision.  A value is held to 2^-62 of its row's largest, so the error of a result is relative to the
+// largest values of two rows and not to each of its terms.  Error of A.X in the norm against quad precision,
+// digits / FP64 tiles: naphthalene .. decacene, (H2O)16, (H2O)40, C20H22 7.1e-17 .. 8.5e-17 / 7.3e-17 ..
+// 1.0e-16; (H2O)24 and two naphthalenes 22 to 1000 bohr apart, each with a random, a unit, a steep and a graded
+// vector, 2.1e-17 .. 1.2e-16 / 2.1e-17 .. 1.8e-16.  The components are as good as the tiles' (medians 5e-17 to
+// 2e-15) but for those 2^-50 and more below their rows' largest: of a unit vector on one of two far fragments,
+// components of 1e-20 keep eight digits or fewer (the tiles: fourteen).  TINCR_GB300_CONTRACTION=fp64 keeps
+// the tiles.
 //
 // What bounds it: 36 digit products per FMA on the tensor cores (2.3 TFLOP of bf16 at 20 vectors of
 // (H2O)128, 1.2 ms at the measured GEMM rate) and the F planes (16 bytes per element, written and read

@@ -10,6 +10,7 @@
 // The value of a product is sum over levels g = s + t <= 7 of G_g 2^(8 (14 - g)) 2^(Ea + Eb - 124) with the level
 // sums G_g of the digit products, i.e. (H 2^32 + L) 2^(Ea + Eb - 68) with H = sum_{g<4} G_g 2^(8 (3 - g)) and
 // L = sum_{g>=4} G_g 2^(8 (7 - g)).
+// Range.  Bounds, digits and results cover all finite doubles; a row with an infinity or a NaN has no digits.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -15,8 +15,9 @@
 // (f64_tile_for).  Every output is one fma chain over ascending k in every tile, so the choice does
 // not change a bit.  Measured against 64x64 alone: S0 + S1 gradient of decacene (n = 192) 79.8 ->
 // 10.2 ms, one A.X product of naphthalene (n = 48) 334 -> 79 us per call, 20 products of (H2O)128
-// (n = 768, 64x64 still chosen for most of it) 55.6 -> 54.4 ms.  Even 16x16 with one output per thread stays pipe-bound: two shared-memory
-// wavefronts and 2 bytes of operands per 16 clocks.
+// kept on the tiles (n = 768, 64x64 still chosen for most of it; large work runs on digits, contract_digits.cu)
+// 55.6 -> 54.4 ms.  Even 16x16 with one output per thread stays pipe-bound: two shared-memory wavefronts and
+// 2 bytes of operands per 16 clocks.
 #pragma once
 
 #include "common.cuh"

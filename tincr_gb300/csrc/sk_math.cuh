@@ -13,7 +13,8 @@
 // ss_sigma, sp_sigma, ps_sigma, pp_pi, pp_sigma (src/param/slako_transformations.rs:57-680).  The
 // gradient with respect to the inter-centre vector r = pos2 - pos1 is
 //     d/dr_c [P(u) V(r)] = (grad_u P . (e_c - u_c u)) V / r + P V'(r) u_c
-// which is the quantity tincr's `slako_transformation_gradients` (:682-6404) hard-codes.
+// which is the quantity tincr's `slako_transformation_gradients` (:682-6404) hard-codes (summed over a pair's
+// block before it is formed: sk_contract in gradient.cu).
 #pragma once
 
 #include <math.h>

@@ -31,7 +31,8 @@ enum Blk { BLK_OCC = 0, BLK_VIRT = 1 };
 // tighter tolerances make a TINCR_PREC_BF16X3 solve finish with FP64 Davidson iterations.
 constexpr double MIXED_TOL_FLOOR = 1e-6;
 
-// FP64 multiply-adds above which the contraction runs as digit GEMMs (contract_digits.cu).  Below, the
+// FP64 multiply-adds of a contraction (all vectors and all products of the call) above which it runs as digit
+// GEMMs (contract_digits.cu).  Below, the
 // twelve launches of that path (about 110 us in all) outweigh the FP64 pipe's 1.7 us per 1e6.  Device
 // time of a call, digits against FP64 tiles: decacene (n = 192) 1 vector, 35e6: 129 / 109 us;
 // pentacene (n = 102) 10 vectors, 53e6: 123 / 149; (H2O)48 (n = 288) 1 vector, 85e6: 148 / 190;
