@@ -10,8 +10,8 @@
 // Fock matrix (up to 8 iterates).  tincr mixes Mulliken charges with Broyden's method and stops at an
 // rms charge change of 1e-5: the same stationary density, reached here to a tighter test.
 //
-// Layout.  A persistent grid of clusters of 1 to 16 CTAs (two CTAs per SM) takes systems from a counter, largest first.
-// A cluster keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and
+// Layout.  A persistent grid of clusters of 1 to 16 CTAs (two CTAs per SM) takes systems from a counter,
+// largest first.  A cluster keeps its system's matrices in a private slot of global memory (a few MB, L2-resident) and
 // runs every step itself; its CTAs share out the tiles, rows, roots and elements of a step and meet at
 // the cluster barrier, small vectors and sums going straight into each other's shared memory:
 //  * the FP64 products of the iterations as exact digit products on warp MMAs (sc_prod); those of small
@@ -24,8 +24,8 @@
 //    pivoting), Loewdin's orthogonalisation to first order (Gram-Schmidt inside clusters of close roots
 //    where that does not do), and the back-transformation by the stored reflections;
 //  * the Fock build, Mulliken charges, DIIS and the energy as element loops and reductions.
-// CTAs per system: sc_ctas_per_system.  Kernel time (ms, LC, to 1e-10) with one CTA per system, FP64 tiles and the eigensolver in every
-// iteration / with clusters / with digit products and purification too:
+// CTAs per system: sc_ctas_per_system.  Kernel time (ms, LC, to 1e-10) with one CTA per system, FP64 tiles and
+// the eigensolver in every iteration / with clusters / with digit products and purification too:
 //     one decacene (192 orbitals)  705 / 123 / 44       128 acene dimers (up to 186)  750 / 417 / 176
 //     16 acene dimers              690 / 160 / 54       64 acenes (up to 102)         145 /  74 /  37
 //     40 acene dimers              719 / 233 / 79       400 acene dimers             1100 / 1081 / 512
@@ -69,7 +69,7 @@ constexpr int SC_SLOTS_PER_SM = 2;
 constexpr int SC_KS = 32;              // k depth of a GEMM slice
 constexpr int SC_DIGITS = 20000;       // n^3 per CTA from which the iterations' FP64 products run on digits
 constexpr int SC_CMAX = 16;            // CTAs per cluster
-constexpr double SC_FILL = 4.0;        // CTAs per SM that a batch of large systems is spread over (twice those that run at once)
+constexpr double SC_FILL = 4.0;        // CTAs per SM that a batch of large systems is spread over (twice what runs at once)
 constexpr double SC_SMALL = 96.0;      // orbitals below which systems count as small (sc_ctas_per_system)
 
 struct ScArgs {
