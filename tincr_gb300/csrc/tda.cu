@@ -605,12 +605,29 @@ void Ctx::set_atoms(int n_atoms_, const int *orbs_per_atom, int n_orb_) {
     upload(stream, d_ao_atom, atom_of.data(), atom_of.size());
 }
 
+void Ctx::swap_atoms_orbitals() {
+    std::swap(n_atoms, tq.n_atoms);
+    std::swap(n_orb, tq.n_orb);
+    std::swap(h_ao_off, tq.h_ao_off);
+    std::swap(d_ao_off, tq.d_ao_off);
+    std::swap(d_ao_atom, tq.d_ao_atom);
+    std::swap(dC, tq.dC);
+    std::swap(dS_, tq.dS_);
+    std::swap(dSC, tq.dSC);
+}
+
 void Ctx::trans_charges(int n_atoms_, const int *opa, int n, const double *C, const double *S, int occ0, int no,
                         int virt0, int nv, double *q_ov, double *q_oo, double *q_vv) {
     if (!C || !S || no <= 0 || nv <= 0 || occ0 < 0 || virt0 < 0 || occ0 + no > n || virt0 + nv > n)
         fail(TINCR_BAD_ARG, "trans_charges: bad orbital ranges");
     check_finite(C, (size_t)n * n, "C");
     check_finite(S, (size_t)n * n, "S");
+    // the set-up system (its sizes, and the orbitals that the gradient reads) stays as it is
+    struct Swapped {
+        Ctx &c;
+        explicit Swapped(Ctx &c_) : c(c_) { c.swap_atoms_orbitals(); }
+        ~Swapped() { c.swap_atoms_orbitals(); }
+    } swapped(*this);
     set_atoms(n_atoms_, opa, n);
     upload_mo(n, C, S);
     struct Job { double *host; int p0, np, q0, nq; };

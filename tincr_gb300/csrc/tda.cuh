@@ -92,6 +92,14 @@ struct Ctx {
     std::vector<double> h_gamma, h_orbe, h_energies;
     int solved_roots = 0;
     DevBuf<double> dS_, d_xyz;
+    // atoms and orbitals of tincr_trans_charges, in the system's place during the call only
+    struct AtomsOrbitals {
+        int n_atoms = 0, n_orb = 0;
+        std::vector<int> h_ao_off;
+        DevBuf<int> d_ao_off, d_ao_atom;
+        DevBuf<double> dC, dS_, dSC;
+    } tq;
+    void swap_atoms_orbitals();
 
     // parameters for the gradient (SK splines, gamma, repulsion)
     bool params_ready = false;
